@@ -615,7 +615,8 @@ extern "C" mth_status mth_create(const mth_params* p, mth_ctx** out) {
   CKC(cudaMalloc(&c->phase_d, P));
   CKC(cudaMalloc(&c->grain_d, sizeof(int) * P));
   CKC(cudaMalloc(&c->eclass_d, sizeof(int) * P));
-  CKC(cudaMalloc(&c->partials, sizeof(double) * 21 * c->nblocks));
+  c->nrows = newton_blocks(c->nv);
+  CKC(cudaMalloc(&c->partials, sizeof(double) * std::max(21LL * c->nblocks, (long long)NPART * c->nrows)));
   CKC(cudaMalloc(&c->red, sizeof(double) * 32));
   CKC(cudaMallocHost(&c->red_h, sizeof(double) * 32));
   CKC(cudaMalloc(&c->bk_d, sizeof(IterBook)));
@@ -764,8 +765,9 @@ IterIn iter_in(const mth_ctx* c) { return IterIn{c->add_d, c->live_d, c->in_batc
 
 // gated: the kernel follows the live flag (inside a batch graph)
 mth_status launch_reduce(mth_ctx* c, int width, bool gated) {
-  LAUNCH(K_REDUCE, 8.0 * width * (c->nblocks + 1),
-         launch_reduce_partials(c->partials, c->nblocks, width, c->red, gated ? iter_in(c) : IterIn{nullptr, nullptr},
+  const int rows = width == NPART ? c->nrows : c->nblocks;   // NPART: the Newton kernels' rows
+  LAUNCH(K_REDUCE, 8.0 * width * (rows + 1),
+         launch_reduce_partials(c->partials, rows, width, c->red, gated ? iter_in(c) : IterIn{nullptr, nullptr},
                                 c->st));
   return MTH_OK;
 }
@@ -975,7 +977,7 @@ mth_status green_iteration(mth_ctx* c) {
   // Newton: read sigma, strain, eps_p (18), rot (9), CRSS (12); write sigma, edot (12);
   // phase (1 B) and elastic class (4 B) per voxel
   LAUNCH(K_NEWTON, (18 + 9 + 12 + 12) * rp + 5.0 * (double)c->nv,
-         launch_newton(c->mixed, c->nc, &f, c->partials, c->nblocks, it, c->st, c->dd));
+         launch_newton(c->mixed, c->nc, &f, c->partials, it, c->st, c->dd));
   return MTH_OK;
 }
 

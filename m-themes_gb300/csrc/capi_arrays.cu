@@ -221,7 +221,8 @@ extern "C" mth_status mth_local_solve(const mth_params* p, const double c066[36]
   cudaStream_t st;
   CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   double *ds, *de, *dst, *dr, *dc, *ded, *der;
-  long long* dit;
+  double* dit;
+  const size_t nb = (size_t)local_solve_blocks((long long)n);
   CK(cudaMalloc(&ds, sizeof(double) * 6 * n));
   CK(cudaMalloc(&de, sizeof(double) * 6 * n));
   CK(cudaMalloc(&dst, sizeof(double) * 6 * n));
@@ -229,32 +230,23 @@ extern "C" mth_status mth_local_solve(const mth_params* p, const double c066[36]
   CK(cudaMalloc(&dc, sizeof(double) * 12 * n));
   CK(cudaMalloc(&ded, sizeof(double) * 6 * n));
   CK(cudaMalloc(&der, sizeof(double) * 2 * n));
-  CK(cudaMalloc(&dit, sizeof(long long) * n));
+  CK(cudaMalloc(&dit, sizeof(double) * nb));
   CK(cudaMemcpyAsync(ds, sig, sizeof(double) * 6 * n, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(de, eps_p, sizeof(double) * 6 * n, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(dst, strain, sizeof(double) * 6 * n, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(dr, rot, sizeof(double) * 9 * n, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(dc, crss, sizeof(double) * 12 * n, cudaMemcpyHostToDevice, st));
-  std::vector<double> rows(n * ETAB_W);
-  for (size_t v = 0; v < n; v++) {
-    class_row(nc.ph[0], rot + 9 * v, &rows[v * ETAB_W]);
-    class_row_add_s0(&rows[v * ETAB_W], sm);
-  }
-  double* det;
-  CK(cudaMalloc(&det, sizeof(double) * rows.size()));
-  CK(cudaMemcpyAsync(det, rows.data(), sizeof(double) * rows.size(), cudaMemcpyHostToDevice, st));
-  CK(launch_local_solve(nc, (long long)n, ds, de, dst, dr, dc, det, ded, der, dit, st));
-  std::vector<long long> it(n);
+  CK(launch_local_solve(nc, (long long)n, ds, de, dst, dr, dc, ded, der, dit, st));
+  std::vector<double> it(nb);
   CK(cudaMemcpyAsync(sig, ds, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(edot, ded, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(err, der, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(it.data(), dit, sizeof(long long) * n, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(it.data(), dit, sizeof(double) * nb, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   long long tot = 0;
-  for (size_t v = 0; v < n; v++) tot += it[v];
+  for (size_t b = 0; b < nb; b++) tot += (long long)it[b];
   if (newton_iters) *newton_iters = tot;
   cudaFree(ds); cudaFree(de); cudaFree(dst); cudaFree(dr); cudaFree(dc); cudaFree(ded); cudaFree(der); cudaFree(dit);
-  cudaFree(det);
   cudaStreamDestroy(st);
   return MTH_OK;
 }

@@ -66,6 +66,7 @@ struct mth_ctx {
   GreenConst gc;
   cudaStream_t st;
   int nblocks;
+  int nrows;          // rows of partial sums the Newton kernels write
   // device memory
   void* fieldmem;
   Fields<float> ff;

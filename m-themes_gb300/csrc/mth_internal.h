@@ -182,17 +182,26 @@ constexpr int NPART_END = 12;  // epsp[6], edot[6]
 
 // law: 0 power law + Voce, 1 dislocation density (per-system constants in
 // Fields::ddc, harden off)
-cudaError_t launch_newton(int mixed, const NewtonConst& nc, const void* fields, double* partials, int nblocks,
-                          const IterIn& it, cudaStream_t st, int law = 0);
+// (the Newton kernels write one row of partial sums per block: newton_blocks rows)
+cudaError_t launch_newton(int mixed, const NewtonConst& nc, const void* fields, double* partials, const IterIn& it,
+                          cudaStream_t st, int law = 0);
+cudaError_t launch_newton_f32(int mixed, const NewtonConst& nc, const Fields<float>& f, double* partials,
+                              const IterIn& it, cudaStream_t st, int law);
+cudaError_t launch_newton_f64(const NewtonConst& nc, const Fields<double>& f, double* partials, const IterIn& it,
+                              cudaStream_t st, int law);
+int newton_threads(long long nv);
+int newton_blocks(long long nv);
 // kernel attributes the Newton launches need, set on the current device
 cudaError_t prepare_newton_kernels();
 cudaError_t launch_end_step(int mixed, const NewtonConst& nc, const void* fields, const double anti_uniform[3],
                             int do_orient, int do_harden, double* partials, int nblocks, cudaStream_t st, int law = 0);
 cudaError_t launch_setup(int mixed, const NewtonConst& nc, const void* fields, const double* euler,
                          const double d6[6], int nblocks, cudaStream_t st);
+// block_iters: the Newton steps of each of the local_solve_blocks(n) blocks
+int local_solve_blocks(long long n);
 cudaError_t launch_local_solve(const NewtonConst& nc, long long n, double* sig, const double* epsp,
-                               const double* strain, const double* rot, const double* crss, const double* etab,
-                               double* edot, double* err, long long* iters, cudaStream_t st);
+                               const double* strain, const double* rot, const double* crss, double* edot, double* err,
+                               double* block_iters, cudaStream_t st);
 // ------------------------------------------------------------ DRX / phase field
 constexpr int PF_K = 16;   // (id, eta) entries a voxel's list holds
 constexpr int PF_NM = 32;  // ids of a voxel's 3x3x3 neighbourhood N(v)

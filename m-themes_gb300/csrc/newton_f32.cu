@@ -1,0 +1,183 @@
+// newton_f32.cu -- the local solve of the FP32 modes (newton.cu describes the
+// problem, local_solve.cuh the iteration).
+#include "newton_dev.cuh"
+
+namespace mth {
+
+__device__ __noinline__ bool solve5_f64(const float* H, const float* b, float* x) {
+  return ldl_solve5_wide<float, double>(H, b, x);
+}
+
+// FP32 modes: one voxel per thread, everything of the solve in FP32 but the
+// systems the refinement leaves to FP64 (local_solve.cuh).  Each thread's
+// K, c and slip-law constants live in its column of shared memory.
+//
+// What bounds it: issue slots (0.70 of the cycles issue; the FP32 pipe is
+// half busy, DRAM a tenth).  128^3, 100 Green iterations, ms (events around
+// each launch): 37.5, against 103.5 for the earlier kernels, whose blocks
+// stepped their solves in lock step to share the FP64 solves; the FP32-solve
+// mode at 64^3 5.2 against 10.7, the dislocation-density law at 96^3 17.9
+// against 31.5.
+template <int SOLVE, int LAW, bool GEN, int MINB>
+__global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_constant__ LocalConst lc,
+                                                                 Fields<float> f, double* __restrict__ partials,
+                                                                 IterIn it) {
+  if (!is_live(it)) return;
+  extern __shared__ __align__(16) float ls_sm[];
+  float* col = ls_sm + threadIdx.x;
+  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long P = f.nv;
+  float acc[NPART];
+#pragma unroll
+  for (int i = 0; i < NPART; i++) acc[i] = 0.0f;
+  if (v < P) {
+    const int jph = f.phase[v];
+    const SlipF& ph = lc.ph[GEN ? jph : 0];
+    if (GEN ? ph.type == 0 : jph == 0) {
+      const float* et = f.etabf + (size_t)f.eclass[v] * ETAB_W;
+      float x[5], ed[5], h, dh, ref2;
+      {
+        float lam[6], u[6], R[9], Q[25];
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+          lam[i] = f.sig[i * P + v];
+          u[i] = f.epsp[i * P + v] - f.strain[i * P + v];
+        }
+#pragma unroll
+        for (int i = 0; i < 9; i++) R[i] = f.rot[i * P + v];
+        // c = Q (eps_p - eps - S0 lambda)
+        h = (lc.s0hh * lam[5] - u[5]) / (lc.s0hh + et[ET_SEL_HH]);
+        dh = h - lam[5];
+        ref2 = lam[5] * lam[5];
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+          float a = lc.s0[i * 5] * lam[0];
+#pragma unroll
+          for (int j = 1; j < 5; j++) a = fmaf(lc.s0[i * 5 + j], lam[j], a);
+          u[i] -= a;
+          ref2 = fmaf(lam[i], lam[i], ref2);
+        }
+        rot_to_q_dev<float>(R, Q);
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+          float a = Q[i * 5] * lam[0], b = Q[i * 5] * u[0];
+#pragma unroll
+          for (int j = 1; j < 5; j++) {
+            a = fmaf(Q[i * 5 + j], lam[j], a);
+            b = fmaf(Q[i * 5 + j], u[j], b);
+          }
+          x[i] = a;
+          ls_at(col, LS_C + i) = b;
+        }
+        float S[15];
+#pragma unroll
+        for (int i = 0; i < 15; i++) S[i] = et[ET_STOT + i];
+        store_k(Q, S, col);
+      }
+      if constexpr (LAW == 0) {
+#pragma unroll
+        for (int s = 0; s < NSYS; s++) {
+          const float t = f.crss[s * P + v];
+          ls_at(col, LS_LAW + s) = t > 0.0f ? rcp_f32(t) : 0.0f;   // 0 in the slots past nsys
+          if (GEN) {
+            const float tb = t + ph.tau_off;
+            ls_at(col, LS_LAW + NSYS + s) = t > 0.0f ? rcp_f32(tb) : 0.0f;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int s = 0; s < 3 * NSYS; s++) ls_at(col, LS_LAW + s) = f.ddc[s * P + v];
+      }
+      const SolveF32 o =
+          solve_f32<SOLVE, LAW, GEN, false>(lc, ph, col, et[ET_STOT_MIN], ref2, h, dh, x, ed);
+      // back to sample axes; the inputs are read again rather than held
+      // through the solve
+      float lam[6], u[6], R[9], ss[5], es[5];
+#pragma unroll
+      for (int i = 0; i < 9; i++) R[i] = ld_again(f.rot + i * P + v);
+      dev_to_sample<float>(R, x, ss);
+      dev_to_sample<float>(R, ed, es);
+#pragma unroll
+      for (int i = 0; i < 6; i++) {
+        lam[i] = ld_again(f.sig + i * P + v);
+        u[i] = ld_again(f.epsp + i * P + v) - ld_again(f.strain + i * P + v);
+      }
+      float cs = dh * dh, ce;
+      {
+        const float de = fmaf(et[ET_SEL_HH], h, u[5]);
+        ce = de * de;
+      }
+#pragma unroll
+      for (int i = 0; i < 5; i++) {
+        const float ds = ss[i] - lam[i];
+        cs = fmaf(ds, ds, cs);
+        float de = fmaf(lc.dt, es[i], u[i]);
+#pragma unroll
+        for (int j = 0; j < 5; j++) de = fmaf(et[ET_SEL + pk5s(i, j)], ss[j], de);
+        ce = fmaf(de, de, ce);
+      }
+#pragma unroll
+      for (int i = 0; i < 5; i++) {
+        f.sig[i * P + v] = ss[i];
+        f.edot[i * P + v] = es[i];
+        acc[2 + i] = ss[i];
+      }
+      f.sig[5 * P + v] = h;
+      f.edot[5 * P + v] = 0.0f;
+      acc[7] = h;
+      acc[0] = sqrtf(cs);
+      acc[1] = sqrtf(ce);
+      if (GEN && jph == 0) {
+#pragma unroll
+        for (int i = 0; i < 6; i++) acc[8 + i] = acc[2 + i];
+      }
+      acc[14] = (float)o.it;   // small integers: exact
+      acc[15] = o.failed ? 1.0f : 0.0f;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 6; i++) {
+        f.sig[i * P + v] = 0.0f;
+        f.edot[i * P + v] = 0.0f;
+      }
+    }
+  }
+  newton_block_sums<float, GEN>(acc, col, partials);
+}
+
+// Blocks of 128 threads per SM the kernels are compiled for.  100 launches,
+// ms: 128^3 37.1 with 4 (128 registers, no spills), 38.8 with 5, 39.6 with 6
+// (80 registers, 280 B of spills); dislocation-density law at 96^3 17.5 with
+// 4, 19.3 with 3, 22.3 with 5.
+#ifndef MTH_F32_MINB
+#define MTH_F32_MINB 4
+#endif
+#ifndef MTH_DD_MINB
+#define MTH_DD_MINB 4
+#endif
+
+template <int SOLVE, int LAW, bool GEN, int MINB>
+static cudaError_t launch_f32(const LocalConst& lc, const Fields<float>& f, double* partials, const IterIn& it,
+                              cudaStream_t st) {
+  const int nt = newton_threads(f.nv);
+  return launch_chain(newton_f32_kernel<SOLVE, LAW, GEN, MINB>, dim3(newton_blocks(f.nv)), dim3(nt),
+                      sizeof(float) * LS_NT * ls_rows<LAW, GEN>(), st, it.pdl, lc, f, partials, it);
+}
+template <int SOLVE, int LAW, int MINB>
+static cudaError_t launch_f32_gen(bool plain, const LocalConst& lc, const Fields<float>& f, double* partials,
+                                  const IterIn& it, cudaStream_t st) {
+  return plain ? launch_f32<SOLVE, LAW, false, MINB>(lc, f, partials, it, st)
+               : launch_f32<SOLVE, LAW, true, MINB>(lc, f, partials, it, st);
+}
+cudaError_t launch_newton_f32(int mixed, const NewtonConst& nc, const Fields<float>& f, double* partials,
+                              const IterIn& it, cudaStream_t st, int law) {
+  LocalConst lc;
+  fill_local(nc, false, lc);
+  const bool plain = plain_phase(nc, lc);
+  // dislocation-density law: refined solves at every step in all mixed modes
+  if (law == 1) return launch_f32_gen<LS_REFINED, 1, MTH_DD_MINB>(nc.ph1_only != 0, lc, f, partials, it, st);
+  if (mixed == 2) return launch_f32_gen<LS_FAST, 0, MTH_F32_MINB>(plain, lc, f, partials, it, st);
+  if (mixed == 3) return launch_f32_gen<LS_NEAR_ROOT, 0, MTH_F32_MINB>(plain, lc, f, partials, it, st);
+  return launch_f32_gen<LS_REFINED, 0, MTH_F32_MINB>(plain, lc, f, partials, it, st);
+}
+
+}  // namespace mth
