@@ -295,6 +295,7 @@ void ctx_free(mth_ctx* c) {
   cudaFree(c->etab_d);
   cudaFree(c->etabf_d);
   cudaFree(c->partials);
+  cudaFree(c->rowsum);
   if (c->red_h) cudaFreeHost(c->red_h);
   cudaFree(c->bk_d);
   if (c->book_h) cudaFreeHost(c->book_h);
@@ -615,8 +616,10 @@ extern "C" mth_status mth_create(const mth_params* p, mth_ctx** out) {
   CKC(cudaMalloc(&c->phase_d, P));
   CKC(cudaMalloc(&c->grain_d, sizeof(int) * P));
   CKC(cudaMalloc(&c->eclass_d, sizeof(int) * P));
-  c->nrows = newton_blocks(c->nv);
+  c->nrows = newton_blocks(c->nv, !c->mixed);
   CKC(cudaMalloc(&c->partials, sizeof(double) * std::max(21LL * c->nblocks, (long long)NPART * c->nrows)));
+  CKC(cudaMalloc(&c->rowsum, iter_end_scratch()));
+  CKC(cudaMemset(c->rowsum, 0, iter_end_scratch()));
   CKC(cudaMalloc(&c->red, sizeof(double) * 32));
   CKC(cudaMallocHost(&c->red_h, sizeof(double) * 32));
   CKC(cudaMalloc(&c->bk_d, sizeof(IterBook)));
@@ -764,16 +767,21 @@ extern "C" mth_status mth_destroy(mth_ctx* c) {
 IterIn iter_in(const mth_ctx* c) { return IterIn{c->add_d, c->live_d, c->in_batch ? 0 : c->pdl}; }
 
 // gated: the kernel follows the live flag (inside a batch graph)
-mth_status launch_reduce(mth_ctx* c, int width, bool gated) {
-  const int rows = width == NPART ? c->nrows : c->nblocks;   // NPART: the Newton kernels' rows
-  LAUNCH(K_REDUCE, 8.0 * width * (rows + 1),
-         launch_reduce_partials(c->partials, rows, width, c->red, gated ? iter_in(c) : IterIn{nullptr, nullptr},
-                                c->st));
+mth_status launch_reduce(mth_ctx* c, int width) {
+  LAUNCH(K_REDUCE, 8.0 * width * (c->nblocks + 1),
+         launch_reduce_partials(c->partials, c->nblocks, width, c->red, IterIn{nullptr, nullptr}, c->st));
+  return MTH_OK;
+}
+
+mth_status iter_end(mth_ctx* c, bool book) {
+  LAUNCH(K_BOOK, 8.0 * NPART * (c->nrows + 1),
+         launch_iter_end(c->partials, c->nrows, c->rowsum, c->red, book ? c->bk_d : nullptr, c->add_d, c->live_d,
+                         iter_in(c), c->st));
   return MTH_OK;
 }
 
 mth_status reduce_to_host(mth_ctx* c, int width, double* out) {
-  mth_status s = launch_reduce(c, width, false);
+  mth_status s = width == NPART ? iter_end(c, false) : launch_reduce(c, width);
   if (s) return s;
   CK(cudaMemcpyAsync(c->red_h, c->red, sizeof(double) * width, cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(c->err_h, c->err_d, sizeof(int), cudaMemcpyDeviceToHost, c->st));
@@ -1354,8 +1362,8 @@ extern "C" mth_status mth_step(mth_ctx* c, mth_step_report* rep) {
   mth_status s = step_begin(c);
   if (s) return s;
   // The iterations run with their bookkeeping on the device (book.cu): each
-  // iteration's kernels, its reduction and the one-warp bookkeeping
-  // kernel, which computes the next iteration's strain increment or drops
+  // iteration's kernels and the one that ends it, which sums the Newton
+  // kernel's rows and computes the next iteration's strain increment or drops
   // the live flag; the host queues groups of iterations and reads the flag
   // once per group, so the iterations follow one another without a host
   // round trip.  Iterations queued after the last one return at once.
@@ -1376,16 +1384,15 @@ extern "C" mth_status mth_step(mth_ctx* c, mth_step_report* rep) {
     return step_end(c, rep);
   }
   CK(cudaMemcpyAsync(c->bk_d, &b, sizeof(IterBook), cudaMemcpyHostToDevice, c->st));
-  LAUNCH(K_BOOK, 0, launch_iter_book(c->bk_d, c->red, c->add_d, c->live_d, 1, c->st, 0));
+  LAUNCH(K_BOOK, 0, launch_book_start(c->bk_d, c->add_d, c->live_d, c->st));
   int queued = 0, group = 2;
   for (;;) {
     const int n = std::min(group, b.iter_max - queued);
     for (int k = 0; k < n; k++) {
       s = c->mixed ? green_iteration<float>(c) : green_iteration<double>(c);
       if (s) return s;
-      s = launch_reduce(c, NPART, true);
+      s = iter_end(c, true);
       if (s) return s;
-      LAUNCH(K_BOOK, 0, launch_iter_book(c->bk_d, c->red, c->add_d, c->live_d, 0, c->st, c->pdl));
     }
     queued += n;
     CK(cudaMemcpyAsync(&c->book_h[0], c->live_d, sizeof(int), cudaMemcpyDeviceToHost, c->st));

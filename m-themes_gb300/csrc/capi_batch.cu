@@ -142,7 +142,7 @@ mth_status tune_passes(const mth_params& p, PassChoice* out) {
 
 // The Green-iteration loop of a mechanical step of every member, as one
 // graph: a while node whose body is one iteration of all members (each
-// member's FFT passes, Newton, reduction and one-warp bookkeeping as a
+// member's FFT passes, Newton and the kernel that ends the iteration as a
 // parallel branch, gated by its live flag) followed by a one-thread kernel
 // that continues the loop while a member is live.  The bookkeeping kernels
 // (book.cu) drop a member's flag when it is done, so one graph launch runs
@@ -195,8 +195,7 @@ mth_status batch_capture(mth_batch* b) {
       c->prof_on = 0;
       c->st = b->branch[i];
       if (!s) s = c->mixed ? green_iteration<float>(c) : green_iteration<double>(c);
-      if (!s) s = launch_reduce(c, NPART, true);
-      if (!s) ck(launch_iter_book(c->bk_d, c->red, c->add_d, c->live_d, 0, c->st, 0));
+      if (!s) s = iter_end(c, true);
       c->st = b->st;
       c->prof_on = prof;
       ck(cudaEventRecord(b->join[i], b->branch[i]));
@@ -332,7 +331,7 @@ extern "C" mth_status mth_batch_step(mth_batch* b, mth_step_report* reports) {
   for (int i = 0; i < n; i++) {
     mth_ctx* c = b->rve[i];
     CK(cudaMemcpyAsync(c->bk_d, &c->bk, sizeof(IterBook), cudaMemcpyHostToDevice, b->st));
-    CK(launch_iter_book(c->bk_d, c->red, c->add_d, c->live_d, 1, b->st, 0));
+    CK(launch_book_start(c->bk_d, c->add_d, c->live_d, b->st));
   }
   CK(cudaMemsetAsync(b->ctl_d, 0, sizeof(int) * 2, b->st));
   CK(cudaGraphLaunch(b->exec, b->st));

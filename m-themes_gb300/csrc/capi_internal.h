@@ -67,6 +67,7 @@ struct mth_ctx {
   cudaStream_t st;
   int nblocks;
   int nrows;          // rows of partial sums the Newton kernels write
+  void* rowsum;       // scratch of their reduction (launch_iter_end)
   // device memory
   void* fieldmem;
   Fields<float> ff;
@@ -190,7 +191,8 @@ const char* prof_class_name(int cls);
 // Phases of a mechanical step (capi.cu), shared by mth_step, the batch
 // driver and the adjoint.
 IterIn iter_in(const mth_ctx* c);
-mth_status launch_reduce(mth_ctx* c, int width, bool gated);
+mth_status launch_reduce(mth_ctx* c, int width);
+mth_status iter_end(mth_ctx* c, bool book);   // the Newton rows' sums, the iteration's bookkeeping
 mth_status reduce_to_host(mth_ctx* c, int width, double* out);
 template <typename T>
 mth_status green_iteration(mth_ctx* c);

@@ -189,8 +189,8 @@ cudaError_t launch_newton_f32(int mixed, const NewtonConst& nc, const Fields<flo
                               const IterIn& it, cudaStream_t st, int law);
 cudaError_t launch_newton_f64(const NewtonConst& nc, const Fields<double>& f, double* partials, const IterIn& it,
                               cudaStream_t st, int law);
-int newton_threads(long long nv);
-int newton_blocks(long long nv);
+int newton_threads(long long nv, bool fp64);
+int newton_blocks(long long nv, bool fp64);
 // kernel attributes the Newton launches need, set on the current device
 cudaError_t prepare_newton_kernels();
 cudaError_t launch_end_step(int mixed, const NewtonConst& nc, const void* fields, const double anti_uniform[3],
@@ -353,9 +353,13 @@ cudaError_t launch_disgrad_skew(int mixed, const void* wspin, void* skew, long l
 cudaError_t launch_reduce_partials(const double* partials, int nblocks, int width, double* out, const IterIn& it,
                                    cudaStream_t st);
 
-// the per-iteration bookkeeping on the device (book.cu, book.cuh)
+// the end of an iteration on the device (book.cu, book.cuh): the Newton
+// kernels' rows summed into red (NPART) and, with b, the bookkeeping; scratch:
+// iter_end_scratch() bytes, zero before the first call
 struct IterBook;
-cudaError_t launch_iter_book(IterBook* b, const double* red, double* add, int* live, int first, cudaStream_t st,
-                             int pdl);
+size_t iter_end_scratch();
+cudaError_t launch_book_start(IterBook* b, double* add, int* live, cudaStream_t st);
+cudaError_t launch_iter_end(const double* rows, int nrows, void* scratch, double* red, IterBook* b, double* add,
+                            int* live, const IterIn& it, cudaStream_t st);
 
 }  // namespace mth

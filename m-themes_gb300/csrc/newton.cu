@@ -29,16 +29,17 @@
 namespace mth {
 
 // ------------------------------------------------------------ Newton kernels
-// Threads per block: 128, or 64 / 32 where that would leave SMs without a
-// block (the solves are long and independent, so a small grid wants its
-// warps spread: 16^3 voxels are 32 blocks of 128 threads on 32 of the 152
-// SMs, or 128 blocks of 32).
-int newton_threads(long long nv) {
+// Threads per block: 128 in FP32 and 64 in FP64, less where that would leave
+// SMs without a block or with one block more than others (the solves are long
+// and independent, so a small grid wants its warps spread: 16^3 voxels are 32
+// blocks of 128 threads on 32 of the 152 SMs, or 128 blocks of 32).
+int newton_threads(long long nv, bool fp64) {
   constexpr long long SMS = 152;
+  if (fp64) return nv >= SMS * 32 * 16 ? 64 : 32;
   return nv >= SMS * 128 * 2 ? 128 : nv >= SMS * 64 * 2 ? 64 : 32;
 }
-int newton_blocks(long long nv) {
-  const int nt = newton_threads(nv);
+int newton_blocks(long long nv, bool fp64) {
+  const int nt = newton_threads(nv, fp64);
   return (int)((nv + nt - 1) / nt);
 }
 

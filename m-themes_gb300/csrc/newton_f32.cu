@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_co
 template <int SOLVE, int LAW, bool GEN, int MINB>
 static cudaError_t launch_f32(const LocalConst& lc, const Fields<float>& f, double* partials, const IterIn& it,
                               cudaStream_t st) {
-  const int nt = newton_threads(f.nv);
-  return launch_chain(newton_f32_kernel<SOLVE, LAW, GEN, MINB>, dim3(newton_blocks(f.nv)), dim3(nt),
+  const int nt = newton_threads(f.nv, false);
+  return launch_chain(newton_f32_kernel<SOLVE, LAW, GEN, MINB>, dim3(newton_blocks(f.nv, false)), dim3(nt),
                       sizeof(float) * LS_NT * ls_rows<LAW, GEN>(), st, it.pdl, lc, f, partials, it);
 }
 template <int SOLVE, int LAW, int MINB>

@@ -1,6 +1,7 @@
 // newton_f64.cu -- the local solve of the FP64 mode and of the array entry
 // points (newton.cu describes the problem).
 #include <atomic>
+#define LS_COLUMNS 64   // threads of the largest block
 #include "newton_dev.cuh"
 
 namespace mth {
@@ -395,7 +396,7 @@ struct FieldIo {
 };
 
 template <int LAW, bool GEN>
-__global__ void __launch_bounds__(LS_NT, 3) newton_f64_kernel(const __grid_constant__ NewtonConst nc,
+__global__ void __launch_bounds__(LS_NT, 6) newton_f64_kernel(const __grid_constant__ NewtonConst nc,
                                                               const __grid_constant__ LocalConst lc,
                                                               const __grid_constant__ Fields<double> f,
                                                               double* __restrict__ partials, IterIn it) {
@@ -457,7 +458,7 @@ static cudaError_t launch_f64(const NewtonConst& nc, const LocalConst& lc, const
                               const IterIn& it, cudaStream_t st) {
   cudaError_t e = f64_opt_in<LAW, GEN>();
   if (e != cudaSuccess) return e;
-  return launch_chain(newton_f64_kernel<LAW, GEN>, dim3(newton_blocks(f.nv)), dim3(newton_threads(f.nv)),
+  return launch_chain(newton_f64_kernel<LAW, GEN>, dim3(newton_blocks(f.nv, true)), dim3(newton_threads(f.nv, true)),
                       f64_smem<LAW, GEN>(), st, it.pdl, nc, lc, f, partials, it);
 }
 
@@ -552,7 +553,7 @@ struct ArrayIo {
 
 // one thread per point; block_iters receives each block's Newton steps
 template <bool GEN>
-__global__ void __launch_bounds__(LS_NT, 3) local_solve_kernel(const __grid_constant__ NewtonConst nc,
+__global__ void __launch_bounds__(LS_NT, 6) local_solve_kernel(const __grid_constant__ NewtonConst nc,
                                                                const __grid_constant__ LocalConst lc, long long n,
                                                                double* sig, const double* __restrict__ epsp,
                                                                const double* __restrict__ strain,
@@ -589,7 +590,7 @@ __global__ void __launch_bounds__(LS_NT, 3) local_solve_kernel(const __grid_cons
   }
 }
 
-int local_solve_blocks(long long n) { return newton_blocks(n); }
+int local_solve_blocks(long long n) { return newton_blocks(n, true); }
 
 cudaError_t launch_local_solve(const NewtonConst& nc, long long n, double* sig, const double* epsp,
                                const double* strain, const double* rot, const double* crss, double* edot, double* err,
@@ -598,7 +599,7 @@ cudaError_t launch_local_solve(const NewtonConst& nc, long long n, double* sig, 
   fill_local(nc, true, lc);
   for (int k = 0; k < 5; k++) lc.s_xt[k] = (float)nc.ph[0].s_xt[k];
   static bool set0[64] = {}, set1[64] = {};
-  const int nb = newton_blocks(n), nt = newton_threads(n);
+  const int nb = newton_blocks(n, true), nt = newton_threads(n, true);
   if (nc.ph[0].tau_back_minus_fwd == 0.0 && lc.ph[0].nm1 > 0) {
     cudaError_t e = smem_opt_in(local_solve_kernel<false>, f64_smem<0, false>(), set0);
     if (e != cudaSuccess) return e;
@@ -621,7 +622,7 @@ cudaError_t launch_local_solve(const NewtonConst& nc, long long n, double* sig, 
 // process exits.  Calls that overlap on the GPU share it and race.
 namespace {
 constexpr long long NOALLOC_MAX_VOXELS = 1LL << 20;
-constexpr int NOALLOC_MAX_BLOCKS = (int)(NOALLOC_MAX_VOXELS / LS_NT);   // smaller blocks only below 38912 points
+constexpr int NOALLOC_MAX_BLOCKS = (int)(NOALLOC_MAX_VOXELS / LS_NT);   // smaller blocks only below 2^17 points
 static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_MAX_BLOCKS + 1];
 
 __global__ void noalloc_total_kernel(double* scratch, int nblocks) {
@@ -661,7 +662,7 @@ cudaError_t launch_local_solve_noalloc(const NewtonConst& nc, long long n, doubl
     if (e != cudaSuccess) return e;
     g_noalloc_ptr[dev].store(scratch, std::memory_order_release);
   }
-  const int nb = newton_blocks(n);
+  const int nb = newton_blocks(n, true);
   // the total slot is the only one read without being written first
   e = cudaMemsetAsync(scratch + NOALLOC_MAX_BLOCKS, 0, sizeof(double), st);
   if (e != cudaSuccess) return e;
