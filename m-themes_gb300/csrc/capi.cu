@@ -880,10 +880,26 @@ extern "C" mth_status mth_upload_microstructure(mth_ctx* c, const int* grain, co
   c->adj_solid = ((size_t)nph1 == n && c->nc.ph[0].type == 0) ? 1 : 0;
   if (!inv6(c->c066, c->s066)) return set_err(MTH_ERR_SINGULAR, "reference stiffness C066 is singular");
   for (size_t k = 0; k < counts.size(); k++) class_row_add_s0(&rows[k * ETAB_W], c->s066);
-  m2t4(c->c066, c->gc.c0);
+  {
+    // acoustic tensor coefficients: A_ik = C_ijkl f_j f_l, the products with
+    // j != l taken together
+    double c4[81];
+    m2t4(c->c066, c4);
+    const int P[6][2] = {{0, 0}, {1, 1}, {2, 2}, {1, 2}, {0, 2}, {0, 1}};
+    auto at = [&](int i, int j, int k, int l) { return c4[((i * 3 + j) * 3 + k) * 3 + l]; };
+    for (int p = 0; p < 6; p++)
+      for (int q = 0; q < 6; q++) {
+        const int i = P[p][0], k = P[p][1], j = P[q][0], l = P[q][1];
+        c->gc.a[p][q] = j == l ? at(i, j, k, l) : at(i, j, k, l) + at(i, l, k, j);
+        c->gc.af[p][q] = (float)c->gc.a[p][q];
+      }
+    for (int i = 0; i < 3; i++) {
+      c->gc.rn[i] = 1.0 / (double)c->n[i];
+      c->gc.rnf[i] = (float)c->gc.rn[i];
+    }
+  }
   for (int i = 0; i < 6; i++)
     for (int j = 0; j < 6; j++) c->gc.s066[i * 6 + j] = c->s066[i][j];
-  for (int i = 0; i < 81; i++) c->gc.c0f[i] = (float)c->gc.c0[i];
   for (int i = 0; i < 36; i++) c->gc.s066f[i] = (float)c->gc.s066[i];
   c->gc.elast_bc = c->p.elast_bc;
   m2t4(c->s066, c->s0_4);

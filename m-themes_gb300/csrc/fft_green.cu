@@ -199,15 +199,19 @@ __global__ void __launch_bounds__(256) fft_x_green_kernel(const GreenConst gc, c
     const int kk = idx % kb;
     const int kx = idx / kb;
     if (k0 + kk >= kzn) continue;
-    c2<T> s[6], a[3];
+    T s[2][6], a[2][3];
 #pragma unroll
-    for (int c = 0; c < 6; c++) s[c] = r[(c * kb + kk) * ls + kx];
-    green_point<T>(gc, kx, y, k0 + kk, n0, n1, n2, s, a);
+    for (int c = 0; c < 6; c++) {
+      const c2<T> v = r[(c * kb + kk) * ls + kx];
+      s[0][c] = v.x;
+      s[1][c] = v.y;
+    }
+    green_point<T, 2>(gc, kx, y, k0 + kk, n0, n1, n2, s, a);
 #pragma unroll
-    for (int c = 0; c < 6; c++) r[(c * kb + kk) * ls + kx] = s[c];
+    for (int c = 0; c < 6; c++) r[(c * kb + kk) * ls + kx] = mk<T>(s[0][c], s[1][c]);
     const long long o = base + kx * S + kk;
 #pragma unroll
-    for (int c = 0; c < 3; c++) anti_acc[c * kplane + o] = cadd<T>(anti_acc[c * kplane + o], a[c]);
+    for (int c = 0; c < 3; c++) anti_acc[c * kplane + o] = cadd<T>(anti_acc[c * kplane + o], mk<T>(a[0][c], a[1][c]));
   }
   __syncthreads();
   c2<T>* r2 = do_fft<T, NC>(r, other, n0, ls, nl, pl, tw_i, +1);

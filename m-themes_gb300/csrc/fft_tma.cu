@@ -204,6 +204,21 @@ constexpr int NT = 256;   // threads per block of every TMA pass
 constexpr int RMAX_Z = 8;     // largest radix: z passes
 constexpr int RMAX_S = 16;    // strided (y, x) and Green passes
 
+// Largest radix of a tile of `lines` lines of L points.  FP32: RMAX_S.  FP64:
+// every warp instruction occupies its sub-partition's FP64 pipe for 64 cycles
+// whatever its active lanes, so the butterflies have to fill warps on all four
+// sub-partitions: the largest radix that leaves at least 64 of them, else 4.
+// Per launch at least 64 / 32 / no such limit: y pass of 32^3 27.0 / 27.2 /
+// 53.6 us (two launches), of 128^3 0.54 / 0.64 / 0.64 ms, x + Green of 48^3
+// 89 / 99 / 99 us.
+template <typename T>
+__host__ __device__ constexpr int rmax_tile(int L, int lines) {
+  if (sizeof(T) == 4) return RMAX_S;
+  for (int r = RMAX_S; r > 4; r /= 2)
+    if (L % r == 0 && L / r * lines >= 64) return r;
+  return 4;
+}
+
 }  // namespace
 
 // Tile parameters, shared with the host launchers.
@@ -336,7 +351,7 @@ __global__ void __launch_bounds__(NT) fft_s_tma_kernel(const __grid_constant__ C
     tma_load4(D, &m, x0, c1, c2i, comp, &bar);
   }
   if (!block_wait_loads(&bar, &ok_s, err)) return;
-  tile_fft<T, L, KB, KB, 0, 1, 1, SG, NT, RMAX_S, false>(D, tw);
+  tile_fft<T, L, KB, KB, 0, 1, 1, SG, NT, rmax_tile<T>(L, KB), false>(D, tw);
   fence_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -385,21 +400,44 @@ __global__ void __launch_bounds__(NT, xg_min_blocks<T, L, KB>()) fft_xg_tma_kern
     for (int c = 0; c < 3; c++) tma_load4(Aq + c * SLAB, &manti, x0, y, 0, c, &bar);
   }
   if (!block_wait_loads(&bar, &ok_s, err)) return;
-  tile_fft<T, L, KB, KB, SLAB, 6, 1, -1, NT, RMAX_S, true>(D, twf);
-  for (int idx = threadIdx.x; idx < SLAB; idx += NT) {
-    const int kk = idx % KB, kx = idx / KB;
-    if (k0 + kk >= kz) continue;
-    c2<T> s[6], a[3];
+  tile_fft<T, L, KB, KB, SLAB, 6, 1, -1, NT, rmax_tile<T>(L, 6 * KB), true>(D, twf);
+  if constexpr (sizeof(T) == 8) {
+    // one thread per wave vector and part: twice the warps for the FP64
+    // operations, which each sub-partition issues at one per 64 cycles
+    for (int i = threadIdx.x; i < 2 * SLAB; i += NT) {
+      const int idx = i >> 1, kk = idx % KB, kx = idx / KB;
+      if (k0 + kk >= kz) continue;
+      T s[1][6], a[1][3];
+      T* Dp = reinterpret_cast<T*>(D) + i;
+      T* Ap = reinterpret_cast<T*>(Aq) + i;
 #pragma unroll
-    for (int c = 0; c < 6; c++) s[c] = D[c * SLAB + idx];
-    green_point<T>(gc, kx, y, k0 + kk, L, n1, n2, s, a);
+      for (int c = 0; c < 6; c++) s[0][c] = Dp[2 * c * SLAB];
+      green_point<T, 1>(gc, kx, y, k0 + kk, L, n1, n2, s, a);
 #pragma unroll
-    for (int c = 0; c < 6; c++) D[c * SLAB + idx] = s[c];
+      for (int c = 0; c < 6; c++) Dp[2 * c * SLAB] = s[0][c];
 #pragma unroll
-    for (int c = 0; c < 3; c++) Aq[c * SLAB + idx] = cadd<T>(Aq[c * SLAB + idx], a[c]);
+      for (int c = 0; c < 3; c++) Ap[2 * c * SLAB] += a[0][c];
+    }
+  } else {
+    for (int idx = threadIdx.x; idx < SLAB; idx += NT) {
+      const int kk = idx % KB, kx = idx / KB;
+      if (k0 + kk >= kz) continue;
+      T s[2][6], a[2][3];
+#pragma unroll
+      for (int c = 0; c < 6; c++) {
+        const c2<T> v = D[c * SLAB + idx];
+        s[0][c] = v.x;
+        s[1][c] = v.y;
+      }
+      green_point<T, 2>(gc, kx, y, k0 + kk, L, n1, n2, s, a);
+#pragma unroll
+      for (int c = 0; c < 6; c++) D[c * SLAB + idx] = mk<T>(s[0][c], s[1][c]);
+#pragma unroll
+      for (int c = 0; c < 3; c++) Aq[c * SLAB + idx] = cadd<T>(Aq[c * SLAB + idx], mk<T>(a[0][c], a[1][c]));
+    }
   }
   __syncthreads();
-  tile_fft<T, L, KB, KB, SLAB, 6, 1, +1, NT, RMAX_S, true>(D, twi);
+  tile_fft<T, L, KB, KB, SLAB, 6, 1, +1, NT, rmax_tile<T>(L, 6 * KB), true>(D, twi);
   fence_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {

@@ -71,10 +71,14 @@ inline cudaError_t launch_chain(void (*k)(KArgs...), dim3 grid, dim3 block, size
 
 // Green-operator constants, passed by value (kernel parameter space).
 struct GreenConst {
-  double c0[81];      // C0_ijkl (chg_basis of C066, src/init.c:376)
+  double a[6][6];     // acoustic tensor from products of the wave vector's components:
+                      // entry (i, k) at row 00, 11, 22, 12, 02, 01 from C0_ijkl
+                      // (chg_basis of C066, src/init.c:376), columns the same pairs (j, l)
   double s066[36];    // S066 = C066^-1 (used at k=0 when ElastBC=0)
-  float c0f[81];      // single-precision copies for the FP32 pass
+  double rn[3];       // 1 / line lengths
+  float af[6][6];     // single-precision copies for the FP32 pass
   float s066f[36];
+  float rnf[3];
   int elast_bc;
 };
 

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) end_step_kernel(const NewtonConst nc, Fie
       for (int i = 0; i < 6; i++) s6[i] = (TF)f.sig[i * P + v];
       typename SlipOf<LAW, TF, TSt>::type slip;
       SlipOf<LAW, TF, TSt>::load(ph, f, v, slip);
-      rot_to_q<TF>(R, Q);
+      rot_to_q_dev<TF>(R, Q);
 #pragma unroll
       for (int i = 0; i < 5; i++) {
         TF a = 0;
