@@ -6,6 +6,7 @@
 // This translation unit is compiled without FMA contraction so that FP64
 // results are the separately rounded operations of the reference, bit for
 // bit.
+#include <climits>
 #include <cstdint>
 #include "mth_common.cuh"
 #include "mth_internal.h"
@@ -167,18 +168,6 @@ __device__ __forceinline__ T pf_read_local(const int* id, const T* ph, int n, in
   if (n > 0 && ph[n - 1] < (T)PF_EPS) return ph[n - 1];
   return (T)0;
 }
-template <typename T>
-__device__ __forceinline__ T pf_read_g(const int* __restrict__ ids, const T* __restrict__ phi,
-                                       const uint8_t* __restrict__ cnt, long long nv, long long w, int j) {
-  const int n = cnt[w];
-  for (int k = 0; k < n; k++)
-    if (ids[(long long)k * nv + w] == j) return phi[(long long)k * nv + w];
-  if (n > 0) {
-    const T t = phi[(long long)(n - 1) * nv + w];
-    if (t < (T)PF_EPS) return t;
-  }
-  return (T)0;
-}
 // PFdata lookup for assignment into a list under construction
 template <typename T>
 __device__ __forceinline__ void pf_write_local(int* id, T* ph, int& n, int j, T val, unsigned* bad) {
@@ -262,12 +251,16 @@ __global__ void __launch_bounds__(256) pf_nlist_kernel(PfView g, const int* __re
 // neighbour is resolved in the pass itself: u(z) = G(z) | (P(z) & u(z-1)),
 // G the voxel's own and its other eight neighbours' part, P whether the
 // z-1 neighbour's flag would carry over, solved for the warp's 32 lanes by
-// a prefix over ballot masks.
+// a prefix over ballot masks.  Passes are queued in groups without a look
+// from the host: pass i counts its changes in chg[i] and returns at once when
+// pass i - 1 counted none (a group of 8 at 128^3: 3 us for an idle pass against
+// 20 us for a host round trip).
 template <typename T>
 __global__ void __launch_bounds__(256) pf_upd_kernel(PfView g, const int* __restrict__ ids, const T* __restrict__ phi,
                                                      const uint8_t* __restrict__ cnt, const int* __restrict__ nid,
                                                      const uint8_t* __restrict__ ncnt, uint8_t* __restrict__ upd,
-                                                     unsigned* __restrict__ word) {
+                                                     unsigned* __restrict__ chg, int pass) {
+  if (pass > 0 && chg[pass - 1] == 0) return;
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool in = v < g.nv;
   const int lane = threadIdx.x & 31;
@@ -307,7 +300,7 @@ __global__ void __launch_bounds__(256) pf_upd_kernel(PfView g, const int* __rest
     const uint8_t u = (uint8_t)((gm >> lane) & 1u);
     if (u != old) {
       upd[v] = u;
-      atomicAdd(&word[0], 1u);
+      chg[pass] = 1;   // any number of writers of the same value
     }
   }
 }
@@ -350,34 +343,106 @@ __global__ void __launch_bounds__(256) pf_tail_kernel(PfView g, const int* __res
 }
 
 // Window averages, one 8x8x8 tile of voxels per block: the tile and its
-// 3-voxel halo (periodic) of initial grain ids, energies and this substep's
-// resets are staged in shared memory once, and every voxel of the tile that
-// updates sums its 7x7x7 window from there, in window order, one pass per
-// held entry.  The window positions before the centre in that order are
-// exactly the voxels earlier in the sweep (the first 171), so a reset applies
-// there when the position lies inside the volume (a periodic image is a halo
-// copy, refreshed only after the sweep).
+// 3-voxel halo (periodic) of initial grain ids and energies are staged in
+// shared memory once, and every voxel of the tile that updates sums its 7x7x7
+// window from there, in window order, up to four held entries in one walk
+// over the window (one walk each took 1.34 ms at 128^3).  The window
+// positions before the centre in that order are exactly the voxels earlier in
+// the sweep (the first 171), so a reset applies there when the position lies
+// inside the volume (a periodic image is a halo copy, refreshed only after
+// the sweep).
+//
+// The first iterate of a substep (ow_prev null) has no resets.  A later one
+// differs only where resets changed: a tile none of whose positions changed
+// its reset returns at once; else the averages that come out different are
+// stored, their voxels marked in vdirty and their ids in idirty, and the
+// value is passed on to the row's summary when this voxel is the row's last
+// writer of the id.
 constexpr int PF_WT = 8;
 constexpr int PF_WH = PF_WT + 6;
+constexpr int PF_WN = PF_WH * PF_WH * PF_WH;
+
+__device__ __forceinline__ unsigned pf_hash(int id) { return ((unsigned)id * 2654435761u) >> 16; }
+// slot of id j >= 1 in row r's table of mask + 1 slots, -1 when absent
+__device__ __forceinline__ int pf_row_find(const int* __restrict__ rw_id, int mask, int r, int j) {
+  const int* t = rw_id + (long long)r * PF_RH;
+  int slot = (int)(pf_hash(j) & (unsigned)mask);
+  for (int tries = 0; tries <= mask; tries++, slot = (slot + 1) & mask) {
+    const int id = t[slot];
+    if (id == j) return slot;
+    if (id == 0) return -1;
+  }
+  return -1;
+}
+// id of held entry k of voxel v (c stored entries)
+__device__ __forceinline__ int pf_held_id(const int* __restrict__ ids, const int* __restrict__ tail, long long nv,
+                                          long long v, int k, int c, int mode) {
+  return (k == c || (mode == 1 && k == c - 1)) ? tail[v] : ids[(long long)k * nv + v];
+}
+
+template <typename T, int W, bool RESET>
+__device__ __forceinline__ void pf_window_sums(const int* __restrict__ s_gid, const T* __restrict__ s_e,
+                                               const uint8_t* __restrict__ s_reset, int base0, const int (&id)[W],
+                                               T (&A)[W], int (&C)[W]) {
+#pragma unroll
+  for (int u = 0; u < W; u++) {
+    A[u] = (T)0;
+    C[u] = 0;
+  }
+  for (int i = 0; i < 7; i++)
+    for (int j = 0; j < 7; j++) {
+      const int base = base0 + (i * PF_WH + j) * PF_WH;
+      const int q0 = (i * 7 + j) * 7;
+#pragma unroll
+      for (int m = 0; m < 7; m++) {
+        const int w = base + m, g = s_gid[w];
+        T e = s_e[w];
+        if (RESET && q0 + m < 171 && s_reset[w]) e = (T)100;
+#pragma unroll
+        for (int u = 0; u < W; u++)
+          if (g == id[u]) {
+            A[u] = A[u] + e;
+            C[u]++;
+          }
+      }
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) pf_window_kernel(PfView g, const int* __restrict__ ids,
                                                         const uint8_t* __restrict__ cnt, const int* __restrict__ tail,
                                                         const uint8_t* __restrict__ tmode, const int* __restrict__ gid0,
                                                         const T* __restrict__ energy, const uint8_t* __restrict__ ow,
-                                                        T* __restrict__ wavg, int tiles_y, int tiles_z) {
-  __shared__ int s_gid[PF_WH * PF_WH * PF_WH];
-  __shared__ T s_e[PF_WH * PF_WH * PF_WH];
-  __shared__ uint8_t s_reset[PF_WH * PF_WH * PF_WH];
+                                                        const uint8_t* __restrict__ ow_prev, T* __restrict__ wavg,
+                                                        const int* __restrict__ rw_id, T* __restrict__ rw_val,
+                                                        const int* __restrict__ rw_zl,
+                                                        const uint8_t* __restrict__ rw_mask,
+                                                        uint8_t* __restrict__ vdirty, uint8_t* __restrict__ idirty,
+                                                        int table_len, int tiles_y, int tiles_z) {
+  __shared__ int s_gid[PF_WN];
+  __shared__ T s_e[PF_WN];
+  __shared__ uint8_t s_reset[PF_WN];
   const int tz = blockIdx.x % tiles_z, ty = (blockIdx.x / tiles_z) % tiles_y, tx = blockIdx.x / (tiles_z * tiles_y);
   const int x0 = tx * PF_WT, y0 = ty * PF_WT, z0 = tz * PF_WT;
-  for (int i = threadIdx.x; i < PF_WH * PF_WH * PF_WH; i += blockDim.x) {
-    const int hz = i % PF_WH, hy = (i / PF_WH) % PF_WH, hx = i / (PF_WH * PF_WH);
-    const int gx = x0 - 3 + hx, gy = y0 - 3 + hy, gz = z0 - 3 + hz;
-    const bool in = gx >= 0 && gx < g.d.n0 && gy >= 0 && gy < g.d.n1 && gz >= 0 && gz < g.d.n2;
-    const long long p = g.d.idx(gx, gy, gz);
+  const bool again = ow_prev != nullptr;
+  if (again) {
+    bool diff = false;
+    for (int i = threadIdx.x; i < PF_WN; i += blockDim.x) {
+      const int gx = x0 - 3 + i / (PF_WH * PF_WH), gy = y0 - 3 + (i / PF_WH) % PF_WH, gz = z0 - 3 + i % PF_WH;
+      uint8_t r = 0;
+      if (gx >= 0 && gx < g.d.n0 && gy >= 0 && gy < g.d.n1 && gz >= 0 && gz < g.d.n2) {
+        const long long p = ((long long)gx * g.d.n1 + gy) * g.d.n2 + gz;
+        r = ow[p];
+        diff |= r != ow_prev[p];
+      }
+      s_reset[i] = r;
+    }
+    if (!__syncthreads_or(diff)) return;
+  }
+  for (int i = threadIdx.x; i < PF_WN; i += blockDim.x) {
+    const long long p = g.d.idx(x0 - 3 + i / (PF_WH * PF_WH), y0 - 3 + (i / PF_WH) % PF_WH, z0 - 3 + i % PF_WH);
     s_gid[i] = gid0[p];
     s_e[i] = energy[p];
-    s_reset[i] = (uint8_t)(in && ow[p]);
   }
   __syncthreads();
   const int lz = threadIdx.x % PF_WT, ly = (threadIdx.x / PF_WT) % PF_WT;
@@ -389,86 +454,113 @@ __global__ void __launch_bounds__(256) pf_window_kernel(PfView g, const int* __r
     const int c = cnt[v], mode = tmode[v];
     const int n = c + (mode == 2 ? 1 : 0);
     if (n <= 1) continue;
-    for (int k = 0; k < n; k++) {
-      const int id = (k == c || (mode == 1 && k == c - 1)) ? tail[v] : ids[(long long)k * g.nv + v];
-      T A = (T)0;
-      int C = 0;
-      int q = 0;
-      for (int i = 0; i < 7; i++)
-        for (int j = 0; j < 7; j++) {
-          const int base = ((lx + i) * PF_WH + (ly + j)) * PF_WH + lz;
-          for (int m = 0; m < 7; m++, q++) {
-            const int w = base + m;
-            if (s_gid[w] == id) {
-              A = A + ((q < 171 && s_reset[w]) ? (T)100 : s_e[w]);
-              C++;
-            }
-          }
+    const int base0 = (lx * PF_WH + ly) * PF_WH + lz;
+    for (int k0 = 0; k0 < n; k0 += 4) {
+      int id[4], C[4];
+      T A[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) id[u] = k0 + u < n ? pf_held_id(ids, tail, g.nv, v, k0 + u, c, mode) : INT_MIN;
+      if (again) {
+        pf_window_sums<T, 4, true>(s_gid, s_e, s_reset, base0, id, A, C);
+      } else if (n - k0 > 2) {
+        pf_window_sums<T, 4, false>(s_gid, s_e, s_reset, base0, id, A, C);
+      } else {
+        int id2[2] = {id[0], id[1]}, C2[2];
+        T A2[2];
+        pf_window_sums<T, 2, false>(s_gid, s_e, s_reset, base0, id2, A2, C2);
+        A[0] = A2[0]; A[1] = A2[1]; A[2] = A[3] = (T)0;
+        C[0] = C2[0]; C[1] = C2[1]; C[2] = C[3] = 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (k0 + u >= n) continue;
+        const T a = C[u] > 0 ? A[u] / (T)C[u] : (T)0;
+        T* out = &wavg[(long long)(k0 + u) * g.nv + v];
+        if (!again) {
+          *out = a;
+        } else if (a != *out) {
+          *out = a;
+          vdirty[v] = 1;
+          if (id[u] >= 1 && id[u] <= table_len) idirty[id[u] - 1] = 1;
+          const int r = x * g.d.n1 + y;
+          const int slot = id[u] >= 1 ? pf_row_find(rw_id, rw_mask[r], r, id[u]) : -1;
+          if (slot >= 0 && rw_zl[(long long)r * PF_RH + slot] == z) rw_val[(long long)r * PF_RH + slot] = a;
         }
-      wavg[(long long)k * g.nv + v] = C > 0 ? A / (T)C : (T)0;
+      }
     }
   }
 }
 
 // Row summaries, one block per row of voxels (x, y): every id the row's
 // updating voxels hold, with the first and last z holding it and the value
-// the last one writes.  Ids go through a shared-memory hash (open addressing,
-// 2 PF_RW slots); the order of the entries is immaterial (lookups are by id).
-constexpr int PF_RHASH = 2 * PF_RW;
+// the last one writes, as a hash table (open addressing, 64 slots, 256 where
+// those fill up), so that a look-up by id takes one or two probes.  The row's
+// bit is set in each id's bitmap of writing rows and the bitmap of that
+// bitmap's words: the latest row before a given one that writes an id is a
+// count of leading zeros away (a prefix of last writers over all blocks of
+// rows, carried forward per substep, took 0.45 ms and the walk to it half of
+// the update's time).
 template <typename T>
 __global__ void __launch_bounds__(128) pf_rows_kernel(PfView g, const int* __restrict__ ids,
                                                       const uint8_t* __restrict__ cnt, const int* __restrict__ tail,
                                                       const uint8_t* __restrict__ tmode, const T* __restrict__ wavg,
                                                       int* __restrict__ rw_id, T* __restrict__ rw_val,
                                                       int* __restrict__ rw_zf, int* __restrict__ rw_zl,
-                                                      uint8_t* __restrict__ rw_n, unsigned* __restrict__ word) {
-  __shared__ int h_id[PF_RHASH], h_zf[PF_RHASH], h_zl[PF_RHASH];
-  __shared__ int h_n;
+                                                      uint8_t* __restrict__ rw_mask, unsigned* __restrict__ bm,
+                                                      unsigned* __restrict__ bl, int bm_w, int bl_w, int table_len,
+                                                      unsigned* __restrict__ word) {
+  __shared__ int h_id[PF_RH], h_zf[PF_RH], h_zl[PF_RH];
+  __shared__ int h_n, h_full;
   const int r = blockIdx.x;
-  for (int i = threadIdx.x; i < PF_RHASH; i += blockDim.x) {
-    h_id[i] = 0;   // grain ids are >= 1 in a table-writing list; 0 marks a free slot
-    h_zf[i] = INT_MAX;
-    h_zl[i] = -1;
-  }
-  if (threadIdx.x == 0) h_n = 0;
-  __syncthreads();
   unsigned bad = 0;
-  // pass 1: slots, first and last z per id
-  for (int z = threadIdx.x; z < g.d.n2; z += blockDim.x) {
-    const long long v = (long long)r * g.d.n2 + z;
-    const int c = cnt[v], mode = tmode[v];
-    const int n = c + (mode == 2 ? 1 : 0);
-    if (n <= 1) continue;
-    for (int k = 0; k < n; k++) {
-      const int id = (k == c || (mode == 1 && k == c - 1)) ? tail[v] : ids[(long long)k * g.nv + v];
-      if (id < 1) { bad |= PF_BAD_TABLE; continue; }
-      int slot = (int)(((unsigned)id * 2654435761u) % PF_RHASH), tries = 0;
-      for (; tries < PF_RHASH; tries++, slot = (slot + 1) % PF_RHASH) {
-        const int prev = atomicCAS(&h_id[slot], 0, id);
-        if (prev == 0) { atomicAdd(&h_n, 1); break; }
-        if (prev == id) break;
-      }
-      if (tries == PF_RHASH) { bad |= PF_BAD_ROW; continue; }
-      atomicMin(&h_zf[slot], z);
-      atomicMax(&h_zl[slot], z);
+  int mask = 63;
+  for (;;) {
+    for (int i = threadIdx.x; i <= mask; i += blockDim.x) {
+      h_id[i] = 0;   // grain ids are >= 1 in a table-writing list; 0 marks a free slot
+      h_zf[i] = INT_MAX;
+      h_zl[i] = -1;
     }
+    if (threadIdx.x == 0) h_n = h_full = 0;
+    __syncthreads();
+    for (int z = threadIdx.x; z < g.d.n2; z += blockDim.x) {
+      const long long v = (long long)r * g.d.n2 + z;
+      const int c = cnt[v], mode = tmode[v];
+      const int n = c + (mode == 2 ? 1 : 0);
+      if (n <= 1) continue;
+      for (int k = 0; k < n; k++) {
+        const int id = pf_held_id(ids, tail, g.nv, v, k, c, mode);
+        if (id < 1) { bad |= PF_BAD_TABLE; continue; }
+        int slot = (int)(pf_hash(id) & (unsigned)mask), tries = 0;
+        for (; tries <= mask; tries++, slot = (slot + 1) & mask) {
+          const int prev = atomicCAS(&h_id[slot], 0, id);
+          if (prev == 0) { atomicAdd(&h_n, 1); break; }
+          if (prev == id) break;
+        }
+        if (tries > mask) { h_full = 1; continue; }
+        atomicMin(&h_zf[slot], z);
+        atomicMax(&h_zl[slot], z);
+      }
+    }
+    __syncthreads();
+    if (mask == 63 && (h_full || h_n > 48)) {
+      mask = PF_RH - 1;
+      __syncthreads();
+      continue;
+    }
+    break;
   }
-  __syncthreads();
-  if (h_n > PF_RW) bad |= PF_BAD_ROW;
-  // pass 2: the last writer's value, compacted into the summary
-  __shared__ int h_pos[PF_RHASH];
-  if (threadIdx.x == 0) {
-    int e = 0;
-    for (int i = 0; i < PF_RHASH; i++) h_pos[i] = (h_id[i] != 0 && e < PF_RW) ? e++ : -1;
-    rw_n[r] = (uint8_t)e;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < PF_RHASH; i += blockDim.x) {
-    const int e = h_pos[i];
-    if (e < 0) continue;
-    rw_id[(long long)e * g.rows + r] = h_id[i];
-    rw_zf[(long long)e * g.rows + r] = h_zf[i];
-    rw_zl[(long long)e * g.rows + r] = h_zl[i];
+  if (h_full || h_n > PF_RW) bad |= PF_BAD_ROW;
+  if (threadIdx.x == 0) rw_mask[r] = (uint8_t)mask;
+  for (int i = threadIdx.x; i <= mask; i += blockDim.x) {
+    const int id = h_id[i];
+    rw_id[(long long)r * PF_RH + i] = id;
+    if (id == 0) continue;
+    rw_zf[(long long)r * PF_RH + i] = h_zf[i];
+    rw_zl[(long long)r * PF_RH + i] = h_zl[i];
+    if (table_len == 0) continue;
+    if (id > table_len) { bad |= PF_BAD_TABLE; continue; }
+    atomicOr(&bm[(long long)(id - 1) * bm_w + (r >> 5)], 1u << (r & 31));
+    atomicOr(&bl[(long long)(id - 1) * bl_w + (r >> 10)], 1u << ((r >> 5) & 31));
   }
   for (int z = threadIdx.x; z < g.d.n2; z += blockDim.x) {
     const long long v = (long long)r * g.d.n2 + z;
@@ -476,79 +568,151 @@ __global__ void __launch_bounds__(128) pf_rows_kernel(PfView g, const int* __res
     const int n = c + (mode == 2 ? 1 : 0);
     if (n <= 1) continue;
     for (int k = 0; k < n; k++) {
-      const int id = (k == c || (mode == 1 && k == c - 1)) ? tail[v] : ids[(long long)k * g.nv + v];
+      const int id = pf_held_id(ids, tail, g.nv, v, k, c, mode);
       if (id < 1) continue;
-      int slot = (int)(((unsigned)id * 2654435761u) % PF_RHASH);
-      for (int tries = 0; tries < PF_RHASH && h_id[slot] != id; tries++) slot = (slot + 1) % PF_RHASH;
-      if (h_id[slot] != id || h_pos[slot] < 0 || h_zl[slot] != z) continue;
-      rw_val[(long long)h_pos[slot] * g.rows + r] = wavg[(long long)k * g.nv + v];
+      int slot = (int)(pf_hash(id) & (unsigned)mask);
+      for (int tries = 0; tries <= mask && h_id[slot] != id; tries++) slot = (slot + 1) & mask;
+      if (h_id[slot] == id && h_zl[slot] == z) rw_val[(long long)r * PF_RH + slot] = wavg[(long long)k * g.nv + v];
     }
   }
   if (bad) atomicOr(&word[1], bad);
 }
 
-// rho_avg of id j as the sweep leaves it just before voxel v: the latest
-// earlier writer in v's row, else in the earlier rows of v's block of PF_RB
-// rows, else the last writer up to the previous block (prefix table), else
-// the table as the previous substep left it
+// the latest row before row r (all rows: r = rows) that writes id j, -1 if none
+__device__ __forceinline__ int pf_row_before(const unsigned* __restrict__ bm, const unsigned* __restrict__ bl, int bm_w,
+                                             int bl_w, int j, int r) {
+  const unsigned* b = bm + (long long)(j - 1) * bm_w;
+  int w = r >> 5;
+  if (r & 31) {
+    const unsigned m = b[w] & ((1u << (r & 31)) - 1u);
+    if (m) return (w << 5) + 31 - __clz(m);
+  }
+  const unsigned* t = bl + (long long)(j - 1) * bl_w;
+  int q = w >> 5;
+  unsigned m = (w & 31) ? t[q] & ((1u << (w & 31)) - 1u) : 0u;
+  while (!m) {
+    if (--q < 0) return -1;
+    m = t[q];
+  }
+  w = (q << 5) + 31 - __clz(m);
+  return (w << 5) + 31 - __clz(b[w]);
+}
+
+// what the look-ups of the rho_avg table read
 template <typename T>
-__device__ T pf_stale(const PfView& g, long long v, int j, const int* __restrict__ ids, const uint8_t* __restrict__ cnt,
-                      const int* __restrict__ tail, const uint8_t* __restrict__ tmode, const T* __restrict__ wavg,
-                      const int* __restrict__ rw_id, const T* __restrict__ rw_val, const int* __restrict__ rw_zf,
-                      const int* __restrict__ rw_zl, const uint8_t* __restrict__ rw_n,
-                      const int* __restrict__ blk_row, const T* __restrict__ blk_val, int table_cap,
-                      const T* __restrict__ table, int table_len, unsigned* bad) {
-  const int r = (int)(v / g.d.n2), z = (int)(v % g.d.n2);
-  // v's row: the summary gives the first and last z holding j
-  const int rn = rw_n[r];
-  for (int e = 0; e < rn; e++) {
-    if (rw_id[(long long)e * g.rows + r] != j) continue;
-    const int zf = rw_zf[(long long)e * g.rows + r], zl = rw_zl[(long long)e * g.rows + r];
-    if (zl < z) return rw_val[(long long)e * g.rows + r];
-    if (zf < z) {   // the latest writer before v lies in [zf, z)
-      for (long long w = v - 1; w >= (long long)r * g.d.n2 + zf; w--) {
-        const int c = cnt[w], m = tmode[w];
-        const int n = c + (m == 2 ? 1 : 0);
-        if (n <= 1) continue;
-        for (int k = 0; k < n; k++) {
-          const int id = (k == c || (m == 1 && k == c - 1)) ? tail[w] : ids[(long long)k * g.nv + w];
-          if (id == j) return wavg[(long long)k * g.nv + w];
+struct PfRows {
+  const int* id;
+  const T* val;
+  const int* zf;
+  const int* zl;
+  const uint8_t* mask;
+  const unsigned* bm;
+  const unsigned* bl;
+  int bm_w, bl_w;
+  const T* table;
+  int table_len;
+};
+
+// rho_avg of id j as the sweep leaves it just before voxel v: the latest
+// earlier writer in v's row, else in the earlier rows, else the table as the
+// previous substep left it
+template <typename T>
+__device__ T pf_stale(const PfView& g, long long v, int r, int z, int j, const int* __restrict__ ids,
+                      const uint8_t* __restrict__ cnt, const int* __restrict__ tail, const uint8_t* __restrict__ tmode,
+                      const T* __restrict__ wavg, const PfRows<T>& rw, unsigned* bad) {
+  if (j >= 1) {
+    const int slot = pf_row_find(rw.id, rw.mask[r], r, j);
+    if (slot >= 0) {
+      const long long at = (long long)r * PF_RH + slot;
+      if (rw.zl[at] < z) return rw.val[at];
+      const int zf = rw.zf[at];
+      if (zf < z) {   // the latest writer before v lies in [zf, z)
+        for (long long w = v - 1; w >= (long long)r * g.d.n2 + zf; w--) {
+          const int c = cnt[w], m = tmode[w];
+          const int n = c + (m == 2 ? 1 : 0);
+          if (n <= 1) continue;
+          for (int k = 0; k < n; k++)
+            if (pf_held_id(ids, tail, g.nv, w, k, c, m) == j) return wavg[(long long)k * g.nv + w];
         }
       }
     }
-    break;
   }
-  if (j < 1 || j > table_len) { *bad |= PF_BAD_TABLE; return (T)0; }
-  const int blk = r / PF_RB;
-  for (int q = r - 1; q >= blk * PF_RB; q--) {
-    const int rn = rw_n[q];
-    for (int e = 0; e < rn; e++)
-      if (rw_id[(long long)e * g.rows + q] == j) return rw_val[(long long)e * g.rows + q];
+  if (j < 1 || j > rw.table_len) { *bad |= PF_BAD_TABLE; return (T)0; }
+  const int q = pf_row_before(rw.bm, rw.bl, rw.bm_w, rw.bl_w, j, r);
+  if (q >= 0) {
+    const int slot = pf_row_find(rw.id, rw.mask[q], q, j);
+    if (slot >= 0) return rw.val[(long long)q * PF_RH + slot];
   }
-  if (blk > 0) {
-    const long long at = (long long)(blk - 1) * table_cap + (j - 1);
-    if (blk_row[at] >= 0) return blk_val[at];
-  }
-  return table[j - 1];
+  return rw.table[j - 1];
 }
 
+// The values of up to four ids at a neighbour (PFdata look-ups by value: the
+// entry's eta, else the weak last entry's, else 0), its list read once
+template <typename T>
+__device__ __forceinline__ void pf_read4(const int* __restrict__ ids, const T* __restrict__ phi,
+                                         const uint8_t* __restrict__ cnt, long long nv, long long w, const int (&j)[4],
+                                         T (&val)[4]) {
+  const int n = cnt[w];
+  T e = (T)0;
+  unsigned hit = 0;
+#pragma unroll
+  for (int u = 0; u < 4; u++) val[u] = (T)0;
+  for (int k = 0; k < n; k++) {
+    const int id = ids[(long long)k * nv + w];
+    e = phi[(long long)k * nv + w];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (id == j[u] && !(hit >> u & 1u)) {
+        val[u] = e;
+        hit |= 1u << u;
+      }
+  }
+  if (n > 0 && e < (T)PF_EPS) {
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (!(hit >> u & 1u)) val[u] = e;
+  }
+}
+
+// New lists.  Four ids of N(v) at a time, so that a neighbour's list is read
+// once for them (a look-up per id and neighbour, each with its own walk over
+// the list, left 6 of 32 lanes active and took 3.4 ms at 128^3 with the table
+// look-ups).  Later iterates of a substep (again) redo a voxel only when one
+// of its averages or a table value it reads changed.
 template <typename T>
 __global__ void __launch_bounds__(128) pf_update_kernel(PfView g, const int* __restrict__ ids, const T* __restrict__ phi,
                                                         const uint8_t* __restrict__ cnt, const int* __restrict__ nid,
                                                         const uint8_t* __restrict__ ncnt, const int* __restrict__ tail,
                                                         const uint8_t* __restrict__ tmode, const T* __restrict__ wavg,
-                                                        const int* __restrict__ rw_id, const T* __restrict__ rw_val,
-                                                        const int* __restrict__ rw_zf, const int* __restrict__ rw_zl,
-                                                        const uint8_t* __restrict__ rw_n, const int* __restrict__ blk_row,
-                                                        const T* __restrict__ blk_val, int table_cap,
-                                                        const T* __restrict__ table, int table_len, int init_gid, T mcoef,
-                                                        T kappa, T mwell, T edisl,
+                                                        PfRows<T> rw, int init_gid, T mcoef, T kappa, T mwell, T edisl,
                                                         const uint8_t* __restrict__ ow_in, uint8_t* __restrict__ ow_out,
-                                                        int* __restrict__ ids2, T* __restrict__ phi2,
-                                                        uint8_t* __restrict__ cnt2, unsigned* __restrict__ word) {
+                                                        int again, const uint8_t* __restrict__ vdirty,
+                                                        const uint8_t* __restrict__ idirty, int* __restrict__ ids2,
+                                                        T* __restrict__ phi2, uint8_t* __restrict__ cnt2,
+                                                        unsigned* __restrict__ word) {
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= g.nv) return;
   const long long nv = g.nv;
+  const int nn = ncnt[v];
+  if (again) {
+    const int c = cnt[v], mode = tmode[v];
+    const int n = c + (mode == 2 ? 1 : 0);
+    bool redo = false;
+    if (n > 1) {
+      redo = vdirty[v] != 0;
+      for (int a = 0; a < nn && !redo; a++) {
+        const int j = nid[(long long)a * nv + v];
+        if (j < 1 || j > rw.table_len || !idirty[j - 1]) continue;
+        bool held = false;
+        for (int k = 0; k < n; k++) held |= pf_held_id(ids, tail, nv, v, k, c, mode) == j;
+        redo = !held;
+      }
+    }
+    if (!redo) {
+      ow_out[v] = ow_in[v];
+      return;
+    }
+  }
   int hid[PF_K + 1];
   T hph[PF_K + 1];
   const int n = pf_held<T>(g, ids, phi, cnt, tail, tmode, v, hid, hph);
@@ -557,10 +721,9 @@ __global__ void __launch_bounds__(128) pf_update_kernel(PfView g, const int* __r
   int on = 0;
   unsigned bad = 0;
   bool reset = false;
-  const int nn = ncnt[v];
   if (n > 1) {
-    const int x = (int)(v / ((long long)g.d.n1 * g.d.n2)), y = (int)((v / g.d.n2) % g.d.n1), z = (int)(v % g.d.n2);
-    const Nbhd nbh(g.d, x, y, z);
+    const int r = (int)(v / g.d.n2), z = (int)(v - (long long)r * g.d.n2);
+    const Nbhd nbh(g.d, r / g.d.n1, r % g.d.n1, z);
     T sum_rex = 0, sum1 = 0, hdef = 0;
     for (int k = 0; k < n; k++) {
       const T a = wavg[(long long)k * nv + v];
@@ -571,34 +734,57 @@ __global__ void __launch_bounds__(128) pf_update_kernel(PfView g, const int* __r
         hdef = hdef + (e * e * e * ((T)10.0 - (T)15.0 * e + (T)6.0 * e * e)) * a;
       }
     }
-    for (int a = 0; a < nn; a++) {
-      const int j = nid[(long long)a * nv + v];
-      const T c = pf_read_local<T>(hid, hph, n, j);
-      const T h = c * c * c * ((T)10.0 - (T)15.0 * c + (T)6.0 * c * c);
-      const T dh = c * c * ((T)30.0 - (T)60.0 * c + (T)30.0 * c * c);
-#define NB(a_, b_, c_) pf_read_g<T>(ids, phi, cnt, nv, nbh.at(a_, b_, c_), j)
-      const T right = NB(1, 0, 0), left = NB(-1, 0, 0), front = NB(0, 1, 0), back = NB(0, -1, 0);
-      const T up = NB(0, 0, 1), down = NB(0, 0, -1);
-      const T lu = NB(-1, 0, 1), ld = NB(-1, 0, -1), lf = NB(-1, -1, 0), lb = NB(-1, 1, 0);
-      const T cuf = NB(0, -1, 1), cub = NB(0, 1, 1), cdf = NB(0, -1, -1), cdb = NB(0, 1, -1);
-      const T ru = NB(1, 0, 1), rdn = NB(1, 0, -1), rf = NB(1, -1, 0), rb = NB(1, 1, 0);
-#undef NB
+    for (int a0 = 0; a0 < nn; a0 += 4) {
+      int j4[4];
+      T s1[4], s2[4], nb[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) j4[u] = a0 + u < nn ? nid[(long long)(a0 + u) * nv + v] : INT_MIN;
+#define PF_SET(s, a_, b_, c_) pf_read4<T>(ids, phi, cnt, nv, nbh.at(a_, b_, c_), j4, s)
+#define PF_ADD(s, a_, b_, c_)      \
+  PF_SET(nb, a_, b_, c_);          \
+  _Pragma("unroll") for (int u = 0; u < 4; u++) s[u] = s[u] + nb[u]
       // laplacian() receives left_up.. as its right_up.. parameters
-      // (src/pf_xrx.c:6-9 against the call at :1193-1198)
-      const T lap = (T)0.5 * (right + left + front + back + up + down) +
-                    (T)0.125 * (cuf + cdf + cub + cdb + ld + lu + lf + lb + ru + rb + rdn + rf) - (T)4.5 * c;
-      T ra;
-      int k = 0;
-      while (k < n && hid[k] != j) k++;
-      if (k < n) ra = wavg[(long long)k * nv + v];
-      else
-        ra = pf_stale<T>(g, v, j, ids, cnt, tail, tmode, wavg, rw_id, rw_val, rw_zf, rw_zl, rw_n, blk_row, blk_val,
-                         table_cap, table, table_len, &bad);
-      if (ra > (T)0) {
-        const T val = c - mcoef * (mwell * (c * c * c - c + (T)3.0 * c * (sum_rex - c * c)) - kappa * lap +
-                                   edisl * dh * ((sum1 - h) * ra - (hdef - h * ra)) / (sum1 * sum1));
-        if (j > init_gid && c < (T)0.5 && val > (T)0.5) reset = true;
-        if (val > (T)PF_KEEP) pf_write_local<T>(oid, oph, on, j, val, &bad);
+      // (src/pf_xrx.c:6-9 against the call at :1193-1198); sums in its order:
+      // right left front back up down, and the twelve edges
+      PF_SET(s1, 1, 0, 0);
+      PF_ADD(s1, -1, 0, 0);
+      PF_ADD(s1, 0, 1, 0);
+      PF_ADD(s1, 0, -1, 0);
+      PF_ADD(s1, 0, 0, 1);
+      PF_ADD(s1, 0, 0, -1);
+      PF_SET(s2, 0, -1, 1);
+      PF_ADD(s2, 0, -1, -1);
+      PF_ADD(s2, 0, 1, 1);
+      PF_ADD(s2, 0, 1, -1);
+      PF_ADD(s2, -1, 0, -1);
+      PF_ADD(s2, -1, 0, 1);
+      PF_ADD(s2, -1, -1, 0);
+      PF_ADD(s2, -1, 1, 0);
+      PF_ADD(s2, 1, 0, 1);
+      PF_ADD(s2, 1, 1, 0);
+      PF_ADD(s2, 1, 0, -1);
+      PF_ADD(s2, 1, -1, 0);
+#undef PF_ADD
+#undef PF_SET
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (a0 + u >= nn) break;
+        const int j = j4[u];
+        const T c = pf_read_local<T>(hid, hph, n, j);
+        const T h = c * c * c * ((T)10.0 - (T)15.0 * c + (T)6.0 * c * c);
+        const T dh = c * c * ((T)30.0 - (T)60.0 * c + (T)30.0 * c * c);
+        const T lap = (T)0.5 * s1[u] + (T)0.125 * s2[u] - (T)4.5 * c;
+        T ra;
+        int k = 0;
+        while (k < n && hid[k] != j) k++;
+        if (k < n) ra = wavg[(long long)k * nv + v];
+        else ra = pf_stale<T>(g, v, r, z, j, ids, cnt, tail, tmode, wavg, rw, &bad);
+        if (ra > (T)0) {
+          const T val = c - mcoef * (mwell * (c * c * c - c + (T)3.0 * c * (sum_rex - c * c)) - kappa * lap +
+                                     edisl * dh * ((sum1 - h) * ra - (hdef - h * ra)) / (sum1 * sum1));
+          if (j > init_gid && c < (T)0.5 && val > (T)0.5) reset = true;
+          if (val > (T)PF_KEEP) pf_write_local<T>(oid, oph, on, j, val, &bad);
+        }
       }
     }
   } else if (n == 1) {
@@ -613,73 +799,19 @@ __global__ void __launch_bounds__(128) pf_update_kernel(PfView g, const int* __r
     phi2[(long long)k * nv + v] = oph[k];
   }
   ow_out[v] = (uint8_t)reset;
-  if ((uint8_t)reset != ow_in[v]) atomicAdd(&word[0], 1u);
+  if ((uint8_t)reset != ow_in[v]) word[0] = 1;   // any number of writers of the same value
   if (bad) atomicOr(&word[1], bad);
 }
 
-// Prefix of the table writers: per block of PF_RB rows and id, the last row
-// writing the id in that block and its value (mark, write), then carried
-// forward over the blocks (prefix), so that entry [b][j] is the last writer
-// of j up to block b.  After the sweep, the last block's entries update the
-// table (final).
-__global__ void pf_blk_mark_kernel(PfView g, const int* __restrict__ rw_id, const uint8_t* __restrict__ rw_n,
-                                   int* __restrict__ blk_row, int table_cap, int table_len,
-                                   unsigned* __restrict__ word) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= g.rows) return;
-  const long long base = (long long)(r / PF_RB) * table_cap;
-  for (int e = 0; e < rw_n[r]; e++) {
-    const int j = rw_id[(long long)e * g.rows + r];
-    if (j < 1 || j > table_len) { atomicOr(&word[1], (unsigned)PF_BAD_TABLE); continue; }
-    atomicMax(&blk_row[base + j - 1], r);
-  }
-}
+// After the sweep, each id's last writer's value into the table.
 template <typename T>
-__global__ void pf_blk_write_kernel(PfView g, const int* __restrict__ rw_id, const T* __restrict__ rw_val,
-                                    const uint8_t* __restrict__ rw_n, const int* __restrict__ blk_row,
-                                    T* __restrict__ blk_val, int table_cap, int table_len) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= g.rows) return;
-  const long long base = (long long)(r / PF_RB) * table_cap;
-  for (int e = 0; e < rw_n[r]; e++) {
-    const int j = rw_id[(long long)e * g.rows + r];
-    if (j >= 1 && j <= table_len && blk_row[base + j - 1] == r) blk_val[base + j - 1] = rw_val[(long long)e * g.rows + r];
-  }
-}
-template <typename T>
-__global__ void pf_blk_prefix_kernel(int nblk, int* __restrict__ blk_row, T* __restrict__ blk_val, int table_cap,
-                                     int table_len) {
+__global__ void pf_table_final_kernel(PfView g, PfRows<T> rw, T* __restrict__ table) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= table_len) return;
-  int cr = blk_row[j];
-  T cv = cr >= 0 ? blk_val[j] : (T)0;
-  // eight blocks' rows loaded before any is written (each address is read
-  // before it is written), then carried forward in order
-  for (int b0 = 1; b0 < nblk; b0 += 8) {
-    int rr[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) rr[u] = b0 + u < nblk ? blk_row[(long long)(b0 + u) * table_cap + j] : 0;
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      if (b0 + u >= nblk) break;
-      const long long at = (long long)(b0 + u) * table_cap + j;
-      if (rr[u] >= 0) {
-        cr = rr[u];
-        cv = blk_val[at];
-      } else if (cr >= 0) {
-        blk_row[at] = cr;
-        blk_val[at] = cv;
-      }
-    }
-  }
-}
-template <typename T>
-__global__ void pf_table_final_kernel(int nblk, const int* __restrict__ blk_row, const T* __restrict__ blk_val,
-                                      int table_cap, int table_len, T* __restrict__ table) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= table_len) return;
-  const long long at = (long long)(nblk - 1) * table_cap + j;
-  if (blk_row[at] >= 0) table[j] = blk_val[at];
+  if (j >= rw.table_len) return;
+  const int q = pf_row_before(rw.bm, rw.bl, rw.bm_w, rw.bl_w, j + 1, g.rows);
+  if (q < 0) return;
+  const int slot = pf_row_find(rw.id, rw.mask[q], q, j + 1);
+  if (slot >= 0) table[j] = rw.val[(long long)q * PF_RH + slot];
 }
 
 // resets applied to the energy; grain id = first maximum, 0 when no eta > 0
@@ -734,7 +866,8 @@ cudaError_t pf_alloc(PfBuffers<T>& b, const int dims[3], int table_len) {
   memset(&b, 0, sizeof(b));
   const long long nv = (long long)dims[0] * dims[1] * dims[2];
   b.rows = dims[0] * dims[1];
-  b.nblk = (b.rows + PF_RB - 1) / PF_RB;
+  b.bm_w = b.rows / 32 + 1;   // a word past the last row, for the look-up from the end
+  b.bl_w = (b.bm_w + 31) / 32 + 1;
   cudaError_t e = cudaSuccess;
   auto get = [&](void** p, size_t bytes) {
     if (e == cudaSuccess) e = cudaMalloc(p, bytes);
@@ -743,9 +876,9 @@ cudaError_t pf_alloc(PfBuffers<T>& b, const int dims[3], int table_len) {
     get((void**)&b.ids[i], sizeof(int) * PF_K * nv);
     get((void**)&b.phi[i], sizeof(T) * PF_K * nv);
     get((void**)&b.cnt[i], (size_t)nv);
-    get((void**)&b.upd[i], (size_t)nv);
     get((void**)&b.ow[i], (size_t)nv);
   }
+  get((void**)&b.upd, (size_t)nv);
   get((void**)&b.gid, sizeof(int) * nv);
   get((void**)&b.energy, sizeof(T) * nv);
   get((void**)&b.nid, sizeof(int) * PF_NM * nv);
@@ -753,12 +886,13 @@ cudaError_t pf_alloc(PfBuffers<T>& b, const int dims[3], int table_len) {
   get((void**)&b.tail, sizeof(int) * nv);
   get((void**)&b.tmode, (size_t)nv);
   get((void**)&b.wavg, sizeof(T) * (PF_K + 1) * nv);
-  get((void**)&b.rw_id, sizeof(int) * PF_RW * (size_t)b.rows);
-  get((void**)&b.rw_val, sizeof(T) * PF_RW * (size_t)b.rows);
-  get((void**)&b.rw_zf, sizeof(int) * PF_RW * (size_t)b.rows);
-  get((void**)&b.rw_zl, sizeof(int) * PF_RW * (size_t)b.rows);
-  get((void**)&b.rw_n, (size_t)b.rows);
-  get((void**)&b.word, sizeof(unsigned) * 2);
+  get((void**)&b.rw_id, sizeof(int) * PF_RH * (size_t)b.rows);
+  get((void**)&b.rw_val, sizeof(T) * PF_RH * (size_t)b.rows);
+  get((void**)&b.rw_zf, sizeof(int) * PF_RH * (size_t)b.rows);
+  get((void**)&b.rw_zl, sizeof(int) * PF_RH * (size_t)b.rows);
+  get((void**)&b.rw_mask, (size_t)b.rows);
+  get((void**)&b.vdirty, (size_t)nv);
+  get((void**)&b.word, sizeof(unsigned) * (2 + PF_UPD_GROUP));
   if (e == cudaSuccess) e = pf_table_reserve(b, table_len, nullptr);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   return e;
@@ -767,11 +901,11 @@ cudaError_t pf_alloc(PfBuffers<T>& b, const int dims[3], int table_len) {
 template <typename T>
 void pf_free(PfBuffers<T>& b) {
   for (int i = 0; i < 2; i++) {
-    cudaFree(b.ids[i]); cudaFree(b.phi[i]); cudaFree(b.cnt[i]); cudaFree(b.upd[i]); cudaFree(b.ow[i]);
+    cudaFree(b.ids[i]); cudaFree(b.phi[i]); cudaFree(b.cnt[i]); cudaFree(b.ow[i]);
   }
-  cudaFree(b.gid); cudaFree(b.energy); cudaFree(b.nid); cudaFree(b.ncnt); cudaFree(b.tail); cudaFree(b.tmode);
-  cudaFree(b.wavg); cudaFree(b.rw_id); cudaFree(b.rw_val); cudaFree(b.rw_zf); cudaFree(b.rw_zl); cudaFree(b.rw_n); cudaFree(b.blk_row);
-  cudaFree(b.blk_val);
+  cudaFree(b.upd); cudaFree(b.gid); cudaFree(b.energy); cudaFree(b.nid); cudaFree(b.ncnt); cudaFree(b.tail); cudaFree(b.tmode);
+  cudaFree(b.wavg); cudaFree(b.rw_id); cudaFree(b.rw_val); cudaFree(b.rw_zf); cudaFree(b.rw_zl); cudaFree(b.rw_mask); cudaFree(b.vdirty);
+  cudaFree(b.bm); cudaFree(b.bl); cudaFree(b.idirty);
   cudaFree(b.table); cudaFree(b.word);
   memset(&b, 0, sizeof(b));
 }
@@ -784,28 +918,31 @@ cudaError_t pf_table_reserve(PfBuffers<T>& b, int len, cudaStream_t st) {
   }
   const int cap = len + 1024;
   T* t = nullptr;
-  int* br = nullptr;
-  T* bv = nullptr;
-  const size_t nb_entries = (size_t)b.nblk * cap;
+  unsigned *bm = nullptr, *bl = nullptr;
+  uint8_t* dirty = nullptr;
   cudaError_t e = cudaMalloc(&t, sizeof(T) * cap);
-  if (e == cudaSuccess) e = cudaMalloc(&br, sizeof(int) * nb_entries);
-  if (e == cudaSuccess) e = cudaMalloc(&bv, sizeof(T) * nb_entries);
+  if (e == cudaSuccess) e = cudaMalloc(&bm, sizeof(unsigned) * (size_t)b.bm_w * cap);
+  if (e == cudaSuccess) e = cudaMalloc(&bl, sizeof(unsigned) * (size_t)b.bl_w * cap);
+  if (e == cudaSuccess) e = cudaMalloc(&dirty, (size_t)cap);
   if (e == cudaSuccess) e = cudaMemsetAsync(t, 0, sizeof(T) * cap, st);
   if (e == cudaSuccess && b.table_cap > 0)
     e = cudaMemcpyAsync(t, b.table, sizeof(T) * b.table_cap, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     cudaFree(t);
-    cudaFree(br);
-    cudaFree(bv);
+    cudaFree(bm);
+    cudaFree(bl);
+    cudaFree(dirty);
     return e;
   }
   cudaFree(b.table);
-  cudaFree(b.blk_row);
-  cudaFree(b.blk_val);
+  cudaFree(b.bm);
+  cudaFree(b.bl);
+  cudaFree(b.idirty);
   b.table = t;
-  b.blk_row = br;
-  b.blk_val = bv;
+  b.bm = bm;
+  b.bl = bl;
+  b.idirty = dirty;
   b.table_cap = b.table_len = cap;
   return cudaSuccess;
 }
@@ -849,53 +986,51 @@ cudaError_t launch_pf_relax(const int dims[3], const int* grain, const T* rho, i
     const T* phi = b.phi[cur];
     const uint8_t* cnt = b.cnt[cur];
     PF_K_LAUNCH(pf_nlist_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.word));
-    // update flags to their fixed point (in place), two passes between
-    // reads of the change counter (a pass at the fixed point changes
-    // nothing, so a second one costs only its launch); the counter read is
-    // the second pass's
-    PF_CK(cudaMemsetAsync(b.upd[0], 0, (size_t)nv, st));
-    const int a = 0;
-    for (long long it = 0; it <= nv; it += 2) {
-      PF_K_LAUNCH(pf_upd_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.upd[a], b.word));
-      PF_CK(cudaMemsetAsync(b.word, 0, sizeof(unsigned), st));
-      PF_K_LAUNCH(pf_upd_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.upd[a], b.word));
-      PF_CK(pf_read_counter(b.word, &changed, st));
+    // update flags to their fixed point (in place), in groups of passes
+    PF_CK(cudaMemsetAsync(b.upd, 0, (size_t)nv, st));
+    for (long long it = 0; it <= nv; it += PF_UPD_GROUP) {
+      unsigned* chg = b.word + 2;
+      PF_CK(cudaMemsetAsync(chg, 0, sizeof(unsigned) * PF_UPD_GROUP, st));
+      for (int k = 0; k < PF_UPD_GROUP; k++)
+        PF_K_LAUNCH(pf_upd_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.upd, chg, k));
+      PF_CK(pf_read_counter(chg + PF_UPD_GROUP - 1, &changed, st));
       if (changed == 0) break;
     }
-    PF_K_LAUNCH(pf_tail_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.upd[a], b.tail,
+    PF_K_LAUNCH(pf_tail_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.upd, b.tail,
                                                                 b.tmode, b.word));
-    // values, with the stored-energy resets to their fixed point
+    // values, with the stored-energy resets to their fixed point; the row
+    // summaries' ids and bitmaps are those of the first iterate
     PF_CK(cudaMemsetAsync(b.ow[0], 0, (size_t)nv, st));
+    const PfRows<T> rw{b.rw_id, b.rw_val, b.rw_zf, b.rw_zl, b.rw_mask, b.bm, b.bl, b.bm_w, b.bl_w, b.table,
+                       b.table_len};
     int o = 0;
     for (long long it = 0; it <= nv; it++) {
       PF_CK(cudaMemsetAsync(b.word, 0, sizeof(unsigned), st));
+      if (it > 0) {
+        PF_CK(cudaMemsetAsync(b.vdirty, 0, (size_t)nv, st));
+        PF_CK(cudaMemsetAsync(b.idirty, 0, (size_t)b.table_cap, st));
+      }
       PF_K_LAUNCH(pf_window_kernel<T><<<wtiles, 256, 0, st>>>(g, ids, cnt, b.tail, b.tmode, grain, b.energy, b.ow[o],
-                                                               b.wavg, wty, wtz));
-      PF_K_LAUNCH(pf_rows_kernel<T><<<g.rows, 128, 0, st>>>(g, ids, cnt, b.tail, b.tmode, b.wavg, b.rw_id, b.rw_val,
-                                                              b.rw_zf, b.rw_zl, b.rw_n, b.word));
-      // prefix of the table writers (their values change over the iterates)
-      PF_CK(cudaMemsetAsync(b.blk_row, 0xff, sizeof(int) * (size_t)b.nblk * b.table_cap, st));
-      if (b.table_len > 0) {
-        PF_K_LAUNCH(pf_blk_mark_kernel<<<nb(g.rows, 256), 256, 0, st>>>(g, b.rw_id, b.rw_n, b.blk_row, b.table_cap,
-                                                                         b.table_len, b.word));
-        PF_K_LAUNCH(pf_blk_write_kernel<T><<<nb(g.rows, 256), 256, 0, st>>>(g, b.rw_id, b.rw_val, b.rw_n, b.blk_row,
-                                                                             b.blk_val, b.table_cap, b.table_len));
-        PF_K_LAUNCH(pf_blk_prefix_kernel<T><<<nb(b.table_len, 128), 128, 0, st>>>(b.nblk, b.blk_row, b.blk_val,
-                                                                                   b.table_cap, b.table_len));
+                                                               it > 0 ? b.ow[1 - o] : nullptr, b.wavg, b.rw_id,
+                                                               b.rw_val, b.rw_zl, b.rw_mask, b.vdirty, b.idirty,
+                                                               b.table_len, wty, wtz));
+      if (it == 0) {
+        PF_CK(cudaMemsetAsync(b.bm, 0, sizeof(unsigned) * (size_t)b.bm_w * b.table_cap, st));
+        PF_CK(cudaMemsetAsync(b.bl, 0, sizeof(unsigned) * (size_t)b.bl_w * b.table_cap, st));
+        PF_K_LAUNCH(pf_rows_kernel<T><<<g.rows, 128, 0, st>>>(g, ids, cnt, b.tail, b.tmode, b.wavg, b.rw_id, b.rw_val,
+                                                              b.rw_zf, b.rw_zl, b.rw_mask, b.bm, b.bl, b.bm_w, b.bl_w,
+                                                              b.table_len, b.word));
       }
       PF_K_LAUNCH(pf_update_kernel<T><<<nb(nv, 128), 128, 0, st>>>(
-          g, ids, phi, cnt, b.nid, b.ncnt, b.tail, b.tmode, b.wavg, b.rw_id, b.rw_val, b.rw_zf, b.rw_zl, b.rw_n,
-          b.blk_row, b.blk_val,
-          b.table_cap, b.table, b.table_len,
-          init_gid, (T)co.mcoef, (T)co.kappa, (T)co.mwell, (T)co.edisl, b.ow[o], b.ow[1 - o], b.ids[1 - cur],
+          g, ids, phi, cnt, b.nid, b.ncnt, b.tail, b.tmode, b.wavg, rw, init_gid, (T)co.mcoef, (T)co.kappa,
+          (T)co.mwell, (T)co.edisl, b.ow[o], b.ow[1 - o], it > 0 ? 1 : 0, b.vdirty, b.idirty, b.ids[1 - cur],
           b.phi[1 - cur], b.cnt[1 - cur], b.word));
       o = 1 - o;
       PF_CK(pf_read_counter(b.word, &changed, st));
       if (changed == 0) break;
     }
     if (b.table_len > 0)
-      PF_K_LAUNCH(pf_table_final_kernel<T><<<nb(b.table_len, 256), 256, 0, st>>>(b.nblk, b.blk_row, b.blk_val,
-                                                                                   b.table_cap, b.table_len, b.table));
+      PF_K_LAUNCH(pf_table_final_kernel<T><<<nb(b.table_len, 256), 256, 0, st>>>(g, rw, b.table));
     cur = 1 - cur;
     PF_K_LAUNCH(pf_finish_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, b.ids[cur], b.phi[cur], b.cnt[cur], b.ow[o],
                                                                   b.energy, b.gid));

@@ -210,7 +210,8 @@ cudaError_t launch_local_solve(const NewtonConst& nc, long long n, double* sig, 
 constexpr int PF_K = 16;   // (id, eta) entries a voxel's list holds
 constexpr int PF_NM = 32;  // ids of a voxel's 3x3x3 neighbourhood N(v)
 constexpr int PF_RW = 128; // ids one row (x, y) of voxels writes to the rho_avg table per substep
-constexpr int PF_RB = 16;  // rows per block of the table-writer prefix
+constexpr int PF_RH = 256; // hash slots of a row's summary
+constexpr int PF_UPD_GROUP = 8;   // passes of the update flags between looks from the host
 
 struct PfCoef { double mcoef, kappa, mwell, edisl; };
 
@@ -229,23 +230,25 @@ struct PfBuffers {
   T* energy;          // stored energy of the call (DefEng_buf), reset to 100 where a recrystallised id passed 0.5
   int* nid;           // N(v) in scan order [PF_NM][nv], and its length
   uint8_t* ncnt;
-  uint8_t* upd[2];    // update flags, fixed-point iterates
+  uint8_t* upd;       // update flags, fixed-point iterates in place
   int* tail;          // id the list's last entry carries when the sweep reaches the voxel
   uint8_t* tmode;     // 0 unchanged, 1 weak last entry relabelled, 2 (tail, 0) appended
   T* wavg;            // window averages of the held entries [PF_K + 1][nv]
   uint8_t* ow[2];     // stored-energy resets of this substep, fixed-point iterates
-  int* rw_id;         // per row: the ids it writes to the table, the last value, and the
-  T* rw_val;          // first and last z of a writer [PF_RW][rows]
+  int* rw_id;         // per row: hash table of the ids it writes to the table, the last value, and the
+  T* rw_val;          // first and last z of a writer [rows][PF_RH]; slots in use: mask + 1
   int* rw_zf;
   int* rw_zl;
-  uint8_t* rw_n;
-  int* blk_row;       // per block of PF_RB rows and table entry: the last row up to that block
-  T* blk_val;         // writing the id, and the value it wrote ([nblk][table_cap]; row -1: none)
+  uint8_t* rw_mask;
+  unsigned* bm;       // per table entry: bitmap of the rows that write it (bm_w words), and of its
+  unsigned* bl;       // words that are not 0 (bl_w words)
+  int bm_w, bl_w;
+  uint8_t* vdirty;    // voxels and table entries whose averages changed in the last iterate
+  uint8_t* idirty;
   T* table;           // rho_avg table: grain id g at g - 1
   int table_len;      // entries the kernels may use (<= table_cap)
   int table_cap;      // entries allocated
-  int nblk;
-  unsigned int* word; // [0] fixed-point change counter, [1] overflow bits
+  unsigned int* word; // [0] fixed-point change flag, [1] overflow bits, [2..] change flags of the update passes
   int cur;            // list buffer holding the result
   int rows;
 };
