@@ -132,7 +132,8 @@ __global__ void paint_apply_kernel(long long nv, int first_id, int* __restrict__
 // passes compute those decisions to their fixed point (iterating until no
 // voxel's decision changes, which happens after at most the length of the
 // longest chain of dependent voxels, in practice two to four iterations):
-//   nlist   N(v): ids with eta > EPSILON over the 3x3x3 block, scan order;
+//   tile    N(v): ids with eta > EPSILON over the 3x3x3 block, scan order, and
+//           the stencil sums of those ids;
 //   upd     whether the voxel holds more than one entry when the sweep
 //           reaches it: it does if it held several, or if it held one strong
 //           entry and one of its nine preceding stencil neighbours that
@@ -168,6 +169,8 @@ __device__ __forceinline__ T pf_read_local(const int* id, const T* ph, int n, in
   if (n > 0 && ph[n - 1] < (T)PF_EPS) return ph[n - 1];
   return (T)0;
 }
+__device__ __forceinline__ unsigned pf_hash(int id) { return ((unsigned)id * 2654435761u) >> 16; }
+
 // PFdata lookup for assignment into a list under construction
 template <typename T>
 __device__ __forceinline__ void pf_write_local(int* id, T* ph, int& n, int j, T val, unsigned* bad) {
@@ -212,35 +215,261 @@ __global__ void pf_init_kernel(PfView g, const int* __restrict__ grain, const T*
   gid[v] = grain[v];
 }
 
+// PFdata look-up by value at voxel w: the entry's eta, else the weak last
+// entry's, else 0
 template <typename T>
-__global__ void __launch_bounds__(256) pf_nlist_kernel(PfView g, const int* __restrict__ ids, const T* __restrict__ phi,
-                                                       const uint8_t* __restrict__ cnt, int* __restrict__ nid,
-                                                       uint8_t* __restrict__ ncnt, unsigned* __restrict__ word) {
-  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= g.nv) return;
-  const int x = (int)(v / ((long long)g.d.n1 * g.d.n2)), y = (int)((v / g.d.n2) % g.d.n1), z = (int)(v % g.d.n2);
-  int L[PF_NM];
-  int n = 0;
+__device__ T pf_read_g(const int* __restrict__ ids, const T* __restrict__ phi, const uint8_t* __restrict__ cnt,
+                       long long nv, long long w, int j) {
+  const int n = cnt[w];
+  T e = (T)0;
+  for (int k = 0; k < n; k++) {
+    e = phi[(long long)k * nv + w];
+    if (ids[(long long)k * nv + w] == j) return e;
+  }
+  return n > 0 && e < (T)PF_EPS ? e : (T)0;
+}
+
+// The stencil in the order laplacian() adds it: it receives left_up.. as its
+// right_up.. parameters (src/pf_xrx.c:6-9 against the call at :1193-1198):
+// right left front back up down, then the twelve edges.
+__constant__ int8_t c_sten[18][3] = {{1, 0, 0},  {-1, 0, 0},  {0, 1, 0},  {0, -1, 0}, {0, 0, 1},  {0, 0, -1},
+                                     {0, -1, 1}, {0, -1, -1}, {0, 1, 1},  {0, 1, -1}, {-1, 0, -1}, {-1, 0, 1},
+                                     {-1, -1, 0}, {-1, 1, 0}, {1, 0, 1},  {1, 1, 0},  {1, 0, -1}, {1, -1, 0}};
+// the stencil's sum without the centre: 0.5 (faces) + 0.125 (edges), from the lists
+template <typename T>
+__device__ T pf_sten_lists(const int* __restrict__ ids, const T* __restrict__ phi, const uint8_t* __restrict__ cnt,
+                           long long nv, const Nbhd& nb, int j) {
+  T s1 = (T)0, s2 = (T)0;
+#pragma unroll 1
+  for (int o = 0; o < 18; o++) {
+    const T e = pf_read_g<T>(ids, phi, cnt, nv, nb.at(c_sten[o][0], c_sten[o][1], c_sten[o][2]), j);
+    if (o < 6) s1 = o == 0 ? e : s1 + e;
+    else s2 = o == 6 ? e : s2 + e;
+  }
+  return (T)0.5 * s1 + (T)0.125 * s2;
+}
+
+// N(v) and the stencil sums of its ids, one 4x8x16 tile of voxels per block.
+// The ids of the tile and its one-voxel halo (about a dozen at a thousand
+// grains in 128^3) get numbers; a position's strong ids are a 64-bit mask of
+// them, so the scan for N(v) tests a word per position and looks into a list
+// only where a new id appears, and the etas are laid out densely in shared
+// memory (missing ids hold what a look-up of them returns), PF_TB ids at a
+// time, so that a stencil term is one load.  (One walk over a neighbour's list
+// per term: 441 million warp instructions a launch at 128^3 for the update, 281
+// million for N(v).)  The sums do not depend on the averages, so the iterates
+// of a substep share them.  sten: PF_NS planes; ids past them, and tiles of
+// more than 64 ids, go through the lists.
+constexpr int PF_TX = 4, PF_TY = 8, PF_TZ = 16, PF_TV = PF_TX * PF_TY * PF_TZ;
+constexpr int PF_HY = PF_TY + 2, PF_HZ = PF_TZ + 2, PF_HN = (PF_TX + 2) * PF_HY * PF_HZ;
+constexpr int PF_TH = 128;   // hash slots
+constexpr int PF_TB = 8;     // ids laid out at a time (ten substeps at 128^3: 24.5 ms, with 12 25.0, with 16 26.5)
+constexpr int PF_NS = 8;
+template <typename T>
+__global__ void __launch_bounds__(256) pf_tile_kernel(PfView g, const int* __restrict__ ids, const T* __restrict__ phi,
+                                                      const uint8_t* __restrict__ cnt, int* __restrict__ nid,
+                                                      uint8_t* __restrict__ ncnt, T* __restrict__ sten, int tiles_y,
+                                                      int tiles_z, unsigned* __restrict__ word) {
+  extern __shared__ __align__(16) unsigned char pf_dyn[];
+  T* dense = reinterpret_cast<T*>(pf_dyn);   // [PF_TB][PF_HN]
+  __shared__ unsigned long long s_mask[PF_HN];
+  __shared__ unsigned s_num[PF_HN];          // numbers of a position's first four entries
+  __shared__ uint8_t s_cnt[PF_HN];
+  __shared__ int s_id[PF_TH], s_of[64];      // hash table, id of a number
+  __shared__ unsigned s_w[PF_HN];            // voxel of a halo position
+  __shared__ uint8_t s_no[PF_TH];            // number of a slot
+  __shared__ int s_n, s_over;
+  const int t = threadIdx.x;
+  const int tz = blockIdx.x % tiles_z, ty = (blockIdx.x / tiles_z) % tiles_y, tx = blockIdx.x / (tiles_z * tiles_y);
+  const int x0 = tx * PF_TX, y0 = ty * PF_TY, z0 = tz * PF_TZ;
+  const long long nv = g.nv;
+  auto voxel_of = [&](int i) { return (long long)s_w[i]; };
+  auto find = [&](int id) {
+    int slot = (int)(pf_hash(id) & (PF_TH - 1));
+    // every id of the tile was inserted, so this ends before the table does
+    for (int tries = 0; tries < PF_TH && s_id[slot] != id; tries++) slot = (slot + 1) & (PF_TH - 1);
+    return (int)s_no[slot];
+  };
+  if (t < PF_TH) s_id[t] = INT_MIN;
+  if (t == 0) s_n = s_over = 0;
+  __syncthreads();
+  for (int i = t; i < PF_HN; i += blockDim.x) {
+    const long long w =
+        g.d.idx(x0 - 1 + i / (PF_HY * PF_HZ), y0 - 1 + (i / PF_HZ) % PF_HY, z0 - 1 + i % PF_HZ);
+    s_w[i] = (unsigned)w;
+    const int c = cnt[w];
+    s_cnt[i] = (uint8_t)c;
+    for (int k = 0; k < c; k++) {
+      const int id = ids[(long long)k * nv + w];
+      int slot = (int)(pf_hash(id) & (PF_TH - 1)), tries = 0;
+      for (; tries < PF_TH; tries++, slot = (slot + 1) & (PF_TH - 1)) {
+        const int prev = s_id[slot] == id ? id : atomicCAS(&s_id[slot], INT_MIN, id);
+        if (prev == INT_MIN || prev == id) break;
+      }
+      if (tries == PF_TH || id == INT_MIN) s_over = 1;
+    }
+  }
+  __syncthreads();
+  if (t < PF_TH && s_id[t] != INT_MIN) {
+    const int no = atomicAdd(&s_n, 1);   // any numbering will do
+    if (no < 64) {
+      s_no[t] = (uint8_t)no;
+      s_of[no] = s_id[t];
+    }
+  }
+  __syncthreads();
+  const int n_ids = s_n;
   unsigned bad = 0;
-  const Nbhd nb(g.d, x, y, z);
-  for (int dx = -1; dx <= 1; dx++)
-    for (int dy = -1; dy <= 1; dy++)
-      for (int dz = -1; dz <= 1; dz++) {
-        const long long w = nb.at(dx, dy, dz);
-        const int c = cnt[w];
+  if (s_over || n_ids > 64) {
+    for (int i = t; i < PF_TV; i += blockDim.x) {
+      const int x = x0 + i / (PF_TY * PF_TZ), y = y0 + (i / PF_TZ) % PF_TY, z = z0 + i % PF_TZ;
+      if (x >= g.d.n0 || y >= g.d.n1 || z >= g.d.n2) continue;
+      const long long v = ((long long)x * g.d.n1 + y) * g.d.n2 + z;
+      const Nbhd nb(g.d, x, y, z);
+      int L[PF_NM];
+      int n = 0;
+      for (int dx = -1; dx <= 1; dx++)
+        for (int dy = -1; dy <= 1; dy++)
+          for (int dz = -1; dz <= 1; dz++) {
+            const long long w = nb.at(dx, dy, dz);
+            const int c = cnt[w];
+            for (int k = 0; k < c; k++) {
+              if (!(phi[(long long)k * nv + w] > (T)PF_EPS)) continue;
+              const int j = ids[(long long)k * nv + w];
+              bool seen = false;
+              for (int a = 0; a < n; a++) seen |= (L[a] == j);
+              if (seen) continue;
+              if (n == PF_NM) { bad |= PF_BAD_NEIGH; continue; }
+              L[n++] = j;
+            }
+          }
+      ncnt[v] = (uint8_t)n;
+      for (int a = 0; a < n; a++) {
+        nid[(long long)a * nv + v] = L[a];
+        if (a < PF_NS) sten[(long long)a * nv + v] = pf_sten_lists<T>(ids, phi, cnt, nv, nb, L[a]);
+      }
+    }
+    if (bad) atomicOr(&word[1], bad);
+    return;
+  }
+  for (int i = t; i < PF_HN; i += blockDim.x) {
+    const long long w = voxel_of(i);
+    const int c = s_cnt[i];
+    unsigned long long m = 0;
+    unsigned num = 0;
+    for (int k = 0; k < c; k++) {
+      const int no = find(ids[(long long)k * nv + w]);
+      if (phi[(long long)k * nv + w] > (T)PF_EPS) m |= 1ull << no;
+      if (k < 4) num |= (unsigned)no << (8 * k);
+    }
+    s_mask[i] = m;
+    s_num[i] = num;
+  }
+  __syncthreads();
+  // N(v): new ids in scan order, then list order
+  unsigned long long mine[2];   // numbers of the first PF_NS ids of this thread's two voxels
+  int mine_n[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int i = t + 256 * h;
+    const int lx = i / (PF_TY * PF_TZ), ly = (i / PF_TZ) % PF_TY, lz = i % PF_TZ;
+    const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
+    mine[h] = 0;
+    mine_n[h] = 0;
+    if (x >= g.d.n0 || y >= g.d.n1 || z >= g.d.n2) continue;
+    const long long v = ((long long)x * g.d.n1 + y) * g.d.n2 + z;
+    unsigned long long seen = 0;
+    int n = 0;
+#pragma unroll 1
+    for (int o = 0; o < 9; o++) {
+      const int q0 = ((lx + o / 3) * PF_HY + ly + o % 3) * PF_HZ + lz;
+#pragma unroll
+      for (int dz = 0; dz < 3; dz++) {
+        const unsigned long long m = s_mask[q0 + dz] & ~seen;
+        if (!m) continue;
+        const int c = s_cnt[q0 + dz];
+        const unsigned num = s_num[q0 + dz];
         for (int k = 0; k < c; k++) {
-          if (!(phi[(long long)k * g.nv + w] > (T)PF_EPS)) continue;
-          const int j = ids[(long long)k * g.nv + w];
-          bool seen = false;
-          for (int a = 0; a < n; a++) seen |= (L[a] == j);
-          if (seen) continue;
+          const int no = k < 4 ? (int)(num >> (8 * k) & 255u) : find(ids[(long long)k * nv + voxel_of(q0 + dz)]);
+          if (!(m >> no & 1ull)) continue;
+          seen |= 1ull << no;
           if (n == PF_NM) { bad |= PF_BAD_NEIGH; continue; }
-          L[n++] = j;
+          nid[(long long)n * nv + v] = s_of[no];
+          if (n < PF_NS) mine[h] |= (unsigned long long)no << (8 * n);
+          n++;
         }
       }
-  ncnt[v] = (uint8_t)n;
-  for (int a = 0; a < n; a++) nid[(long long)a * g.nv + v] = L[a];
+    }
+    ncnt[v] = (uint8_t)n;
+    mine_n[h] = min(n, PF_NS);
+  }
   if (bad) atomicOr(&word[1], bad);
+  for (int b0 = 0; b0 < n_ids; b0 += PF_TB) {
+    const int nb = min(PF_TB, n_ids - b0);
+    __syncthreads();
+    for (int i = t; i < PF_HN; i += blockDim.x) {
+      const long long w = voxel_of(i);
+      const int c = s_cnt[i];
+      const unsigned num = s_num[i];
+      T miss = (T)0;
+      if (c > 0) {
+        const T e = phi[(long long)(c - 1) * nv + w];
+        if (e < (T)PF_EPS) miss = e;
+      }
+      for (int q = 0; q < nb; q++) dense[q * PF_HN + i] = miss;
+      for (int k = 0; k < c; k++) {
+        const int no = (k < 4 ? (int)(num >> (8 * k) & 255u) : find(ids[(long long)k * nv + w])) - b0;
+        if (no >= 0 && no < nb) dense[no * PF_HN + i] = phi[(long long)k * nv + w];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int i = t + 256 * h;
+      const int lx = i / (PF_TY * PF_TZ), ly = (i / PF_TZ) % PF_TY, lz = i % PF_TZ;
+      const long long v = ((long long)(x0 + lx) * g.d.n1 + (y0 + ly)) * g.d.n2 + (z0 + lz);
+      const int at = ((lx + 1) * PF_HY + ly + 1) * PF_HZ + lz + 1;
+      for (int a = 0; a < mine_n[h]; a++) {
+        const int no = (int)(mine[h] >> (8 * a) & 255u) - b0;
+        if (no < 0 || no >= nb) continue;
+        const T* e = dense + no * PF_HN + at;
+        constexpr int DX = PF_HY * PF_HZ, DY = PF_HZ;
+        const T s1 = e[DX] + e[-DX] + e[DY] + e[-DY] + e[1] + e[-1];
+        const T s2 = e[-DY + 1] + e[-DY - 1] + e[DY + 1] + e[DY - 1] + e[-DX - 1] + e[-DX + 1] + e[-DX - DY] +
+                     e[-DX + DY] + e[DX + 1] + e[DX + DY] + e[DX - 1] + e[DX - DY];
+        sten[(long long)a * nv + v] = (T)0.5 * s1 + (T)0.125 * s2;
+      }
+    }
+  }
+}
+
+// What a voxel's update flag depends on: PF_GEN when it updates whatever its
+// neighbours do (it holds several entries), else bit o when the o-th preceding
+// neighbour (c_pred), if it updates, appends an id here: the voxel holds one
+// strong entry and the neighbour's N has an id besides it.
+constexpr unsigned PF_GEN = 1u << 15;
+template <typename T>
+__global__ void __launch_bounds__(256) pf_pred_kernel(PfView g, const int* __restrict__ ids, const T* __restrict__ phi,
+                                                      const uint8_t* __restrict__ cnt, const int* __restrict__ nid,
+                                                      const uint8_t* __restrict__ ncnt,
+                                                      unsigned short* __restrict__ pred) {
+  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= g.nv) return;
+  const int c = cnt[v];
+  unsigned m = c > 1 ? PF_GEN : 0u;
+  if (c == 1 && phi[v] >= (T)PF_EPS) {
+    const int X = ids[v];
+    const int x = (int)(v / ((long long)g.d.n1 * g.d.n2)), y = (int)((v / g.d.n2) % g.d.n1), z = (int)(v % g.d.n2);
+#pragma unroll
+    for (int o = 0; o < 9; o++) {
+      const int qx = x + c_pred[o][0], qy = y + c_pred[o][1], qz = z + c_pred[o][2];
+      if (qx < 0 || qy < 0 || qy >= g.d.n1 || qz < 0 || qz >= g.d.n2) continue;
+      const long long q = ((long long)qx * g.d.n1 + qy) * g.d.n2 + qz;
+      const int nq = ncnt[q];
+      if (nq >= 2 || (nq == 1 && nid[q] != X)) m |= 1u << o;
+    }
+  }
+  pred[v] = (unsigned short)m;
 }
 
 // One pass of the update flags' fixed point, in place.  The flags only turn
@@ -255,42 +484,29 @@ __global__ void __launch_bounds__(256) pf_nlist_kernel(PfView g, const int* __re
 // from the host: pass i counts its changes in chg[i] and returns at once when
 // pass i - 1 counted none (a group of 8 at 128^3: 3 us for an idle pass against
 // 20 us for a host round trip).
-template <typename T>
-__global__ void __launch_bounds__(256) pf_upd_kernel(PfView g, const int* __restrict__ ids, const T* __restrict__ phi,
-                                                     const uint8_t* __restrict__ cnt, const int* __restrict__ nid,
-                                                     const uint8_t* __restrict__ ncnt, uint8_t* __restrict__ upd,
-                                                     unsigned* __restrict__ chg, int pass) {
+__global__ void __launch_bounds__(256) pf_upd_kernel(PfView g, const unsigned short* __restrict__ pred,
+                                                     uint8_t* __restrict__ upd, unsigned* __restrict__ chg, int pass) {
   if (pass > 0 && chg[pass - 1] == 0) return;
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool in = v < g.nv;
   const int lane = threadIdx.x & 31;
-  bool gen = false, prop = false, zin = false;
   uint8_t old = 0;
+  unsigned m = 0;
   if (in) {
     old = upd[v];
-    const int c = cnt[v];
-    gen = c > 1;
-    if (c == 1 && phi[v] >= (T)PF_EPS) {
-      const int X = ids[v];
-      const int x = (int)(v / ((long long)g.d.n1 * g.d.n2)), y = (int)((v / g.d.n2) % g.d.n1), z = (int)(v % g.d.n2);
-      for (int o = 0; o < 9; o++) {
-        const int qx = x + c_pred[o][0], qy = y + c_pred[o][1], qz = z + c_pred[o][2];
-        if (qx < 0 || qy < 0 || qy >= g.d.n1 || qz < 0 || qz >= g.d.n2) continue;
-        const long long q = ((long long)qx * g.d.n1 + qy) * g.d.n2 + qz;
-        const int nq = ncnt[q];
-        const bool carries = nq >= 2 || (nq == 1 && nid[q] != X);
-        if (o == 0) {   // (0,0,-1): the previous voxel of the row
-          prop = carries;
-          zin = upd[q] != 0;
-        } else if (carries && upd[q]) {
-          gen = true;
-        }
-      }
-    }
+    m = old ? PF_GEN : pred[v];
   }
+  bool gen = (m & PF_GEN) != 0;
+  const bool prop = (m & 1u) != 0;   // (0,0,-1): the previous voxel of the row
+  // a set bit's neighbour lies inside the volume, so its index needs no check
+#pragma unroll
+  for (int o = 1; o < 9; o++)
+    if (!gen && (m >> o & 1u))
+      gen = upd[v + ((long long)c_pred[o][0] * g.d.n1 + c_pred[o][1]) * g.d.n2 + c_pred[o][2]] != 0;
+  const bool zin = lane == 0 && prop && upd[v - 1] != 0;
   // u = G | (P & u(z-1)) over the warp; lane 0 takes u(z-1) from the buffer
   const unsigned am = __activemask();
-  unsigned gm = __ballot_sync(am, gen || (lane == 0 && prop && zin)), pm = __ballot_sync(am, prop);
+  unsigned gm = __ballot_sync(am, gen || zin), pm = __ballot_sync(am, prop);
 #pragma unroll
   for (int s = 1; s < 32; s <<= 1) {
     gm |= pm & (gm << s);
@@ -300,9 +516,12 @@ __global__ void __launch_bounds__(256) pf_upd_kernel(PfView g, const int* __rest
     const uint8_t u = (uint8_t)((gm >> lane) & 1u);
     if (u != old) {
       upd[v] = u;
-      chg[pass] = 1;   // any number of writers of the same value
     }
   }
+  // one store per warp, and none once the flag is seen set (a store per voxel
+  // made the pass in which most flags turn on 0.25 ms)
+  const bool changed = in && (uint8_t)((gm >> lane) & 1u) != old;
+  if (__ballot_sync(am, changed) && lane == __ffs((int)am) - 1 && *(volatile unsigned*)&chg[pass] == 0) chg[pass] = 1;
 }
 
 template <typename T>
@@ -362,7 +581,6 @@ constexpr int PF_WT = 8;
 constexpr int PF_WH = PF_WT + 6;
 constexpr int PF_WN = PF_WH * PF_WH * PF_WH;
 
-__device__ __forceinline__ unsigned pf_hash(int id) { return ((unsigned)id * 2654435761u) >> 16; }
 // slot of id j >= 1 in row r's table of mask + 1 slots, -1 when absent
 __device__ __forceinline__ int pf_row_find(const int* __restrict__ rw_id, int mask, int r, int j) {
   const int* t = rw_id + (long long)r * PF_RH;
@@ -398,12 +616,25 @@ __device__ __forceinline__ void pf_window_sums(const int* __restrict__ s_gid, co
         const int w = base + m, g = s_gid[w];
         T e = s_e[w];
         if (RESET && q0 + m < 171 && s_reset[w]) e = (T)100;
+        if constexpr (sizeof(T) == 8) {
+          // at most one of the ids matches: one FP64 addition, to the selected sum
+          T a = (T)0;
 #pragma unroll
-        for (int u = 0; u < W; u++)
-          if (g == id[u]) {
-            A[u] = A[u] + e;
-            C[u]++;
+          for (int u = 0; u < W; u++) a = g == id[u] ? A[u] : a;
+          a = a + e;
+#pragma unroll
+          for (int u = 0; u < W; u++) {
+            A[u] = g == id[u] ? a : A[u];
+            C[u] += g == id[u];
           }
+        } else {
+#pragma unroll
+          for (int u = 0; u < W; u++)
+            if (g == id[u]) {
+              A[u] = A[u] + e;
+              C[u]++;
+            }
+        }
       }
     }
 }
@@ -445,15 +676,35 @@ __global__ void __launch_bounds__(256) pf_window_kernel(PfView g, const int* __r
     s_e[i] = energy[p];
   }
   __syncthreads();
-  const int lz = threadIdx.x % PF_WT, ly = (threadIdx.x / PF_WT) % PF_WT;
-  for (int half = 0; half < 2; half++) {
-    const int lx = threadIdx.x / (PF_WT * PF_WT) + 4 * half;
-    const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
+  // the voxels that update, those with up to two entries from the front of
+  // the list and those with more from its end, so that a warp's voxels take
+  // the same walk (by voxel, half of the lanes idled)
+  __shared__ unsigned short s_list[PF_WT * PF_WT * PF_WT];
+  __shared__ int s_n2, s_n4;
+  if (threadIdx.x == 0) s_n2 = s_n4 = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < PF_WT * PF_WT * PF_WT; i += blockDim.x) {
+    const int x = x0 + i / (PF_WT * PF_WT), y = y0 + (i / PF_WT) % PF_WT, z = z0 + i % PF_WT;
     if (x >= g.d.n0 || y >= g.d.n1 || z >= g.d.n2) continue;
+    const long long v = ((long long)x * g.d.n1 + y) * g.d.n2 + z;
+    const int n = cnt[v] + (tmode[v] == 2 ? 1 : 0);
+    if (n <= 1) continue;
+    if (n == 2) s_list[atomicAdd(&s_n2, 1)] = (unsigned short)i;
+    else s_list[PF_WT * PF_WT * PF_WT - 1 - atomicAdd(&s_n4, 1)] = (unsigned short)i;
+  }
+  __syncthreads();
+  const int n2 = s_n2, n4 = s_n4;
+  // whole warps of each kind
+  const int w2 = (n2 + 31) & ~31, all = w2 + n4;
+  for (int e = threadIdx.x; e < all; e += blockDim.x) {
+    const bool four = e >= w2;
+    if (!four && e >= n2) continue;
+    const int i = four ? s_list[PF_WT * PF_WT * PF_WT - 1 - (e - w2)] : s_list[e];
+    const int lx = i / (PF_WT * PF_WT), ly = (i / PF_WT) % PF_WT, lz = i % PF_WT;
+    const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
     const long long v = ((long long)x * g.d.n1 + y) * g.d.n2 + z;
     const int c = cnt[v], mode = tmode[v];
     const int n = c + (mode == 2 ? 1 : 0);
-    if (n <= 1) continue;
     const int base0 = (lx * PF_WH + ly) * PF_WH + lz;
     for (int k0 = 0; k0 < n; k0 += 4) {
       int id[4], C[4];
@@ -462,7 +713,7 @@ __global__ void __launch_bounds__(256) pf_window_kernel(PfView g, const int* __r
       for (int u = 0; u < 4; u++) id[u] = k0 + u < n ? pf_held_id(ids, tail, g.nv, v, k0 + u, c, mode) : INT_MIN;
       if (again) {
         pf_window_sums<T, 4, true>(s_gid, s_e, s_reset, base0, id, A, C);
-      } else if (n - k0 > 2) {
+      } else if (four) {
         pf_window_sums<T, 4, false>(s_gid, s_e, s_reset, base0, id, A, C);
       } else {
         int id2[2] = {id[0], id[1]}, C2[2];
@@ -613,27 +864,52 @@ struct PfRows {
   int table_len;
 };
 
+// A row's ids and, per id, the bitmap of the z that hold it, in shared memory
+struct PfRowBits {
+  const int* id;          // mask + 1 slots
+  const unsigned* bits;   // words per slot: (n2 + 31) / 32; null: not built
+  int mask, words;
+};
+
 // rho_avg of id j as the sweep leaves it just before voxel v: the latest
 // earlier writer in v's row, else in the earlier rows, else the table as the
 // previous substep left it
 template <typename T>
 __device__ T pf_stale(const PfView& g, long long v, int r, int z, int j, const int* __restrict__ ids,
                       const uint8_t* __restrict__ cnt, const int* __restrict__ tail, const uint8_t* __restrict__ tmode,
-                      const T* __restrict__ wavg, const PfRows<T>& rw, unsigned* bad) {
+                      const T* __restrict__ wavg, const PfRows<T>& rw, const PfRowBits& rb, unsigned* bad) {
+  auto held_at = [&](long long w, T* out) {
+    const int c = cnt[w], m = tmode[w];
+    const int n = c + (m == 2 ? 1 : 0);
+    if (n <= 1) return false;
+    for (int k = 0; k < n; k++)
+      if (pf_held_id(ids, tail, g.nv, w, k, c, m) == j) {
+        *out = wavg[(long long)k * g.nv + w];
+        return true;
+      }
+    return false;
+  };
   if (j >= 1) {
-    const int slot = pf_row_find(rw.id, rw.mask[r], r, j);
-    if (slot >= 0) {
-      const long long at = (long long)r * PF_RH + slot;
-      if (rw.zl[at] < z) return rw.val[at];
-      const int zf = rw.zf[at];
-      if (zf < z) {   // the latest writer before v lies in [zf, z)
-        for (long long w = v - 1; w >= (long long)r * g.d.n2 + zf; w--) {
-          const int c = cnt[w], m = tmode[w];
-          const int n = c + (m == 2 ? 1 : 0);
-          if (n <= 1) continue;
-          for (int k = 0; k < n; k++)
-            if (pf_held_id(ids, tail, g.nv, w, k, c, m) == j) return wavg[(long long)k * g.nv + w];
-        }
+    T a;
+    if (rb.bits) {
+      int slot = (int)(pf_hash(j) & (unsigned)rb.mask), tries = 0;
+      for (; tries <= rb.mask && rb.id[slot] != j; tries++, slot = (slot + 1) & rb.mask)
+        if (rb.id[slot] == 0) tries = rb.mask + 1;
+      if (tries <= rb.mask) {
+        const unsigned* b = rb.bits + slot * rb.words;
+        int w = z >> 5;
+        unsigned m = b[w] & ((1u << (z & 31)) - 1u);
+        while (!m && --w >= 0) m = b[w];
+        if (m && held_at(v - z + (w << 5) + 31 - __clz(m), &a)) return a;
+      }
+    } else {
+      const int slot = pf_row_find(rw.id, rw.mask[r], r, j);
+      if (slot >= 0) {
+        const long long at = (long long)r * PF_RH + slot;
+        if (rw.zl[at] < z) return rw.val[at];
+        const int zf = rw.zf[at];
+        for (long long w = v - 1; w >= v - z + zf; w--)   // the latest writer before v lies in [zf, z)
+          if (held_at(w, &a)) return a;
       }
     }
   }
@@ -646,53 +922,64 @@ __device__ T pf_stale(const PfView& g, long long v, int r, int z, int j, const i
   return rw.table[j - 1];
 }
 
-// The values of up to four ids at a neighbour (PFdata look-ups by value: the
-// entry's eta, else the weak last entry's, else 0), its list read once
-template <typename T>
-__device__ __forceinline__ void pf_read4(const int* __restrict__ ids, const T* __restrict__ phi,
-                                         const uint8_t* __restrict__ cnt, long long nv, long long w, const int (&j)[4],
-                                         T (&val)[4]) {
-  const int n = cnt[w];
-  T e = (T)0;
-  unsigned hit = 0;
-#pragma unroll
-  for (int u = 0; u < 4; u++) val[u] = (T)0;
-  for (int k = 0; k < n; k++) {
-    const int id = ids[(long long)k * nv + w];
-    e = phi[(long long)k * nv + w];
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-      if (id == j[u] && !(hit >> u & 1u)) {
-        val[u] = e;
-        hit |= 1u << u;
-      }
-  }
-  if (n > 0 && e < (T)PF_EPS) {
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-      if (!(hit >> u & 1u)) val[u] = e;
-  }
-}
-
-// New lists.  Four ids of N(v) at a time, so that a neighbour's list is read
-// once for them (a look-up per id and neighbour, each with its own walk over
-// the list, left 6 of 32 lanes active and took 3.4 ms at 128^3 with the table
-// look-ups).  Later iterates of a substep (again) redo a voxel only when one
-// of its averages or a table value it reads changed.
+// New lists, one row of voxels (or, where rows are shorter than a block,
+// several) per block.  The row's own earlier writers come from bitmaps in
+// shared memory (the walk back along the row was half of the kernel's time).
+// Later iterates of a substep (again) redo a voxel only when one of its
+// averages or a table value it reads changed.  128^3, ms per launch: 3.4 before
+// the tables, tiles and bitmaps, now 0.41 for a first iterate and 0.1 to 0.3
+// for a later one.
 template <typename T>
 __global__ void __launch_bounds__(128) pf_update_kernel(PfView g, const int* __restrict__ ids, const T* __restrict__ phi,
                                                         const uint8_t* __restrict__ cnt, const int* __restrict__ nid,
-                                                        const uint8_t* __restrict__ ncnt, const int* __restrict__ tail,
+                                                        const uint8_t* __restrict__ ncnt, const T* __restrict__ sten,
+                                                        const int* __restrict__ tail,
                                                         const uint8_t* __restrict__ tmode, const T* __restrict__ wavg,
                                                         PfRows<T> rw, int init_gid, T mcoef, T kappa, T mwell, T edisl,
                                                         const uint8_t* __restrict__ ow_in, uint8_t* __restrict__ ow_out,
                                                         int again, const uint8_t* __restrict__ vdirty,
                                                         const uint8_t* __restrict__ idirty, int* __restrict__ ids2,
                                                         T* __restrict__ phi2, uint8_t* __restrict__ cnt2,
-                                                        unsigned* __restrict__ word) {
-  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= g.nv) return;
+                                                        int per, int words, unsigned* __restrict__ word) {
+  extern __shared__ int s_rows[];   // per row: PF_RH ids, PF_RH x words bits
   const long long nv = g.nv;
+  const int lr = per > 1 ? threadIdx.x / g.d.n2 : 0;
+  const int r = blockIdx.x * per + lr;
+  const bool in = lr < per && r < g.rows;
+  PfRowBits rb{nullptr, nullptr, 0, words};
+  if (words) {
+    const int row_ints = PF_RH * (1 + words);
+    for (int q = 0; q < per && blockIdx.x * per + q < g.rows; q++) {
+      const int rq = blockIdx.x * per + q, mask = rw.mask[rq];
+      int* t = s_rows + q * row_ints;
+      for (int i = threadIdx.x; i <= mask; i += blockDim.x) t[i] = rw.id[(long long)rq * PF_RH + i];
+      for (int i = threadIdx.x; i < (mask + 1) * words; i += blockDim.x) t[PF_RH + i] = 0;
+    }
+    __syncthreads();
+    if (in) {
+      int* t = s_rows + lr * row_ints;
+      rb.id = t;
+      rb.bits = reinterpret_cast<unsigned*>(t + PF_RH);
+      rb.mask = rw.mask[r];
+      for (int z = per > 1 ? threadIdx.x - lr * g.d.n2 : threadIdx.x; z < g.d.n2; z += per > 1 ? g.d.n2 : blockDim.x) {
+        const long long w = (long long)r * g.d.n2 + z;
+        const int c = cnt[w], mode = tmode[w];
+        const int n = c + (mode == 2 ? 1 : 0);
+        if (n <= 1) continue;
+        for (int k = 0; k < n; k++) {
+          const int id = pf_held_id(ids, tail, nv, w, k, c, mode);
+          if (id < 1) continue;
+          int slot = (int)(pf_hash(id) & (unsigned)rb.mask);
+          for (int tries = 0; tries <= rb.mask && t[slot] != id; tries++) slot = (slot + 1) & rb.mask;
+          if (t[slot] == id) atomicOr(reinterpret_cast<unsigned*>(t + PF_RH) + slot * words + (z >> 5), 1u << (z & 31));
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (!in) return;
+  for (int z = per > 1 ? threadIdx.x - lr * g.d.n2 : threadIdx.x; z < g.d.n2; z += per > 1 ? g.d.n2 : blockDim.x) {
+  const long long v = (long long)r * g.d.n2 + z;
   const int nn = ncnt[v];
   if (again) {
     const int c = cnt[v], mode = tmode[v];
@@ -710,7 +997,7 @@ __global__ void __launch_bounds__(128) pf_update_kernel(PfView g, const int* __r
     }
     if (!redo) {
       ow_out[v] = ow_in[v];
-      return;
+      continue;
     }
   }
   int hid[PF_K + 1];
@@ -722,8 +1009,6 @@ __global__ void __launch_bounds__(128) pf_update_kernel(PfView g, const int* __r
   unsigned bad = 0;
   bool reset = false;
   if (n > 1) {
-    const int r = (int)(v / g.d.n2), z = (int)(v - (long long)r * g.d.n2);
-    const Nbhd nbh(g.d, r / g.d.n1, r % g.d.n1, z);
     T sum_rex = 0, sum1 = 0, hdef = 0;
     for (int k = 0; k < n; k++) {
       const T a = wavg[(long long)k * nv + v];
@@ -734,57 +1019,24 @@ __global__ void __launch_bounds__(128) pf_update_kernel(PfView g, const int* __r
         hdef = hdef + (e * e * e * ((T)10.0 - (T)15.0 * e + (T)6.0 * e * e)) * a;
       }
     }
-    for (int a0 = 0; a0 < nn; a0 += 4) {
-      int j4[4];
-      T s1[4], s2[4], nb[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) j4[u] = a0 + u < nn ? nid[(long long)(a0 + u) * nv + v] : INT_MIN;
-#define PF_SET(s, a_, b_, c_) pf_read4<T>(ids, phi, cnt, nv, nbh.at(a_, b_, c_), j4, s)
-#define PF_ADD(s, a_, b_, c_)      \
-  PF_SET(nb, a_, b_, c_);          \
-  _Pragma("unroll") for (int u = 0; u < 4; u++) s[u] = s[u] + nb[u]
-      // laplacian() receives left_up.. as its right_up.. parameters
-      // (src/pf_xrx.c:6-9 against the call at :1193-1198); sums in its order:
-      // right left front back up down, and the twelve edges
-      PF_SET(s1, 1, 0, 0);
-      PF_ADD(s1, -1, 0, 0);
-      PF_ADD(s1, 0, 1, 0);
-      PF_ADD(s1, 0, -1, 0);
-      PF_ADD(s1, 0, 0, 1);
-      PF_ADD(s1, 0, 0, -1);
-      PF_SET(s2, 0, -1, 1);
-      PF_ADD(s2, 0, -1, -1);
-      PF_ADD(s2, 0, 1, 1);
-      PF_ADD(s2, 0, 1, -1);
-      PF_ADD(s2, -1, 0, -1);
-      PF_ADD(s2, -1, 0, 1);
-      PF_ADD(s2, -1, -1, 0);
-      PF_ADD(s2, -1, 1, 0);
-      PF_ADD(s2, 1, 0, 1);
-      PF_ADD(s2, 1, 1, 0);
-      PF_ADD(s2, 1, 0, -1);
-      PF_ADD(s2, 1, -1, 0);
-#undef PF_ADD
-#undef PF_SET
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        if (a0 + u >= nn) break;
-        const int j = j4[u];
-        const T c = pf_read_local<T>(hid, hph, n, j);
-        const T h = c * c * c * ((T)10.0 - (T)15.0 * c + (T)6.0 * c * c);
-        const T dh = c * c * ((T)30.0 - (T)60.0 * c + (T)30.0 * c * c);
-        const T lap = (T)0.5 * s1[u] + (T)0.125 * s2[u] - (T)4.5 * c;
-        T ra;
-        int k = 0;
-        while (k < n && hid[k] != j) k++;
-        if (k < n) ra = wavg[(long long)k * nv + v];
-        else ra = pf_stale<T>(g, v, r, z, j, ids, cnt, tail, tmode, wavg, rw, &bad);
-        if (ra > (T)0) {
-          const T val = c - mcoef * (mwell * (c * c * c - c + (T)3.0 * c * (sum_rex - c * c)) - kappa * lap +
-                                     edisl * dh * ((sum1 - h) * ra - (hdef - h * ra)) / (sum1 * sum1));
-          if (j > init_gid && c < (T)0.5 && val > (T)0.5) reset = true;
-          if (val > (T)PF_KEEP) pf_write_local<T>(oid, oph, on, j, val, &bad);
-        }
+    for (int a = 0; a < nn; a++) {
+      const int j = nid[(long long)a * nv + v];
+      const T c = pf_read_local<T>(hid, hph, n, j);
+      const T h = c * c * c * ((T)10.0 - (T)15.0 * c + (T)6.0 * c * c);
+      const T dh = c * c * ((T)30.0 - (T)60.0 * c + (T)30.0 * c * c);
+      const T st = a < PF_NS ? sten[(long long)a * nv + v]
+                             : pf_sten_lists<T>(ids, phi, cnt, nv, Nbhd(g.d, r / g.d.n1, r % g.d.n1, z), j);
+      const T lap = st - (T)4.5 * c;
+      T ra;
+      int k = 0;
+      while (k < n && hid[k] != j) k++;
+      if (k < n) ra = wavg[(long long)k * nv + v];
+      else ra = pf_stale<T>(g, v, r, z, j, ids, cnt, tail, tmode, wavg, rw, rb, &bad);
+      if (ra > (T)0) {
+        const T val = c - mcoef * (mwell * (c * c * c - c + (T)3.0 * c * (sum_rex - c * c)) - kappa * lap +
+                                   edisl * dh * ((sum1 - h) * ra - (hdef - h * ra)) / (sum1 * sum1));
+        if (j > init_gid && c < (T)0.5 && val > (T)0.5) reset = true;
+        if (val > (T)PF_KEEP) pf_write_local<T>(oid, oph, on, j, val, &bad);
       }
     }
   } else if (n == 1) {
@@ -801,6 +1053,7 @@ __global__ void __launch_bounds__(128) pf_update_kernel(PfView g, const int* __r
   ow_out[v] = (uint8_t)reset;
   if ((uint8_t)reset != ow_in[v]) word[0] = 1;   // any number of writers of the same value
   if (bad) atomicOr(&word[1], bad);
+  }
 }
 
 // After the sweep, each id's last writer's value into the table.
@@ -879,10 +1132,12 @@ cudaError_t pf_alloc(PfBuffers<T>& b, const int dims[3], int table_len) {
     get((void**)&b.ow[i], (size_t)nv);
   }
   get((void**)&b.upd, (size_t)nv);
+  get((void**)&b.pred, sizeof(unsigned short) * nv);
   get((void**)&b.gid, sizeof(int) * nv);
   get((void**)&b.energy, sizeof(T) * nv);
   get((void**)&b.nid, sizeof(int) * PF_NM * nv);
   get((void**)&b.ncnt, (size_t)nv);
+  get((void**)&b.sten, sizeof(T) * PF_NS * nv);
   get((void**)&b.tail, sizeof(int) * nv);
   get((void**)&b.tmode, (size_t)nv);
   get((void**)&b.wavg, sizeof(T) * (PF_K + 1) * nv);
@@ -903,7 +1158,7 @@ void pf_free(PfBuffers<T>& b) {
   for (int i = 0; i < 2; i++) {
     cudaFree(b.ids[i]); cudaFree(b.phi[i]); cudaFree(b.cnt[i]); cudaFree(b.ow[i]);
   }
-  cudaFree(b.upd); cudaFree(b.gid); cudaFree(b.energy); cudaFree(b.nid); cudaFree(b.ncnt); cudaFree(b.tail); cudaFree(b.tmode);
+  cudaFree(b.upd); cudaFree(b.pred); cudaFree(b.gid); cudaFree(b.energy); cudaFree(b.nid); cudaFree(b.ncnt); cudaFree(b.sten); cudaFree(b.tail); cudaFree(b.tmode);
   cudaFree(b.wavg); cudaFree(b.rw_id); cudaFree(b.rw_val); cudaFree(b.rw_zf); cudaFree(b.rw_zl); cudaFree(b.rw_mask); cudaFree(b.vdirty);
   cudaFree(b.bm); cudaFree(b.bl); cudaFree(b.idirty);
   cudaFree(b.table); cudaFree(b.word);
@@ -981,18 +1236,34 @@ cudaError_t launch_pf_relax(const int dims[3], const int* grain, const T* rho, i
   unsigned changed = 0;
   const int wtx = (dims[0] + PF_WT - 1) / PF_WT, wty = (dims[1] + PF_WT - 1) / PF_WT, wtz = (dims[2] + PF_WT - 1) / PF_WT;
   const int wtiles = wtx * wty * wtz;
+  const int ntx = (dims[0] + PF_TX - 1) / PF_TX, nty = (dims[1] + PF_TY - 1) / PF_TY,
+            ntz = (dims[2] + PF_TZ - 1) / PF_TZ;
+  const int ntiles = ntx * nty * ntz;
+  const size_t tsm = sizeof(T) * PF_TB * PF_HN;
+  PF_CK(cudaFuncSetAttribute(pf_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
+  // the update's rows per 128-thread block, and the words of a row's bitmaps:
+  // none (the walk along the row) where they would pass 48 KB, z lines over 1408
+  const int uper = dims[2] >= 128 ? 1 : 128 / dims[2];
+  int uwords = (dims[2] + 31) / 32;
+  size_t usm = sizeof(int) * (size_t)uper * PF_RH * (1 + uwords);
+  if (usm > 47 * 1024) {
+    uwords = 0;
+    usm = 0;
+  }
   for (int s = 0; s < substeps; s++) {
     const int* ids = b.ids[cur];
     const T* phi = b.phi[cur];
     const uint8_t* cnt = b.cnt[cur];
-    PF_K_LAUNCH(pf_nlist_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.word));
+    PF_K_LAUNCH(pf_tile_kernel<T><<<ntiles, 256, tsm, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.sten, nty, ntz,
+                                                            b.word));
     // update flags to their fixed point (in place), in groups of passes
+    PF_K_LAUNCH(pf_pred_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.pred));
     PF_CK(cudaMemsetAsync(b.upd, 0, (size_t)nv, st));
     for (long long it = 0; it <= nv; it += PF_UPD_GROUP) {
       unsigned* chg = b.word + 2;
       PF_CK(cudaMemsetAsync(chg, 0, sizeof(unsigned) * PF_UPD_GROUP, st));
       for (int k = 0; k < PF_UPD_GROUP; k++)
-        PF_K_LAUNCH(pf_upd_kernel<T><<<nb(nv, 256), 256, 0, st>>>(g, ids, phi, cnt, b.nid, b.ncnt, b.upd, chg, k));
+        PF_K_LAUNCH(pf_upd_kernel<<<nb(nv, 256), 256, 0, st>>>(g, b.pred, b.upd, chg, k));
       PF_CK(pf_read_counter(chg + PF_UPD_GROUP - 1, &changed, st));
       if (changed == 0) break;
     }
@@ -1021,10 +1292,10 @@ cudaError_t launch_pf_relax(const int dims[3], const int* grain, const T* rho, i
                                                               b.rw_zf, b.rw_zl, b.rw_mask, b.bm, b.bl, b.bm_w, b.bl_w,
                                                               b.table_len, b.word));
       }
-      PF_K_LAUNCH(pf_update_kernel<T><<<nb(nv, 128), 128, 0, st>>>(
-          g, ids, phi, cnt, b.nid, b.ncnt, b.tail, b.tmode, b.wavg, rw, init_gid, (T)co.mcoef, (T)co.kappa,
+      PF_K_LAUNCH(pf_update_kernel<T><<<nb(g.rows, uper), 128, usm, st>>>(
+          g, ids, phi, cnt, b.nid, b.ncnt, b.sten, b.tail, b.tmode, b.wavg, rw, init_gid, (T)co.mcoef, (T)co.kappa,
           (T)co.mwell, (T)co.edisl, b.ow[o], b.ow[1 - o], it > 0 ? 1 : 0, b.vdirty, b.idirty, b.ids[1 - cur],
-          b.phi[1 - cur], b.cnt[1 - cur], b.word));
+          b.phi[1 - cur], b.cnt[1 - cur], uper, uwords, b.word));
       o = 1 - o;
       PF_CK(pf_read_counter(b.word, &changed, st));
       if (changed == 0) break;

@@ -230,6 +230,8 @@ struct PfBuffers {
   T* energy;          // stored energy of the call (DefEng_buf), reset to 100 where a recrystallised id passed 0.5
   int* nid;           // N(v) in scan order [PF_NM][nv], and its length
   uint8_t* ncnt;
+  T* sten;            // stencil sums of the first ids of N(v)
+  unsigned short* pred;   // what each update flag depends on
   uint8_t* upd;       // update flags, fixed-point iterates in place
   int* tail;          // id the list's last entry carries when the sweep reaches the voxel
   uint8_t* tmode;     // 0 unchanged, 1 weak last entry relabelled, 2 (tail, 0) appended
