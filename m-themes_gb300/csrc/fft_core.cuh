@@ -22,23 +22,31 @@ __host__ __device__ constexpr int ct_radix(int n, int idx) {
   return 1;
 }
 
-// Plans of the in-register tile FFTs (fft_tma.cu): the largest radix up to
-// RMAX first (16, 8, 4, then 2, then 3), so a line needs fewer stages, each
-// one pair of block-wide synchronisations.
+// Plans of the in-register tile FFTs (fft_tma.cuh): the fewest stages with
+// radices up to rmax (each stage is a pair of block-wide synchronisations and
+// a round trip through shared memory), of those the one whose largest radix is
+// smallest (more butterflies to spread over the threads), largest radix first.
+__host__ __device__ constexpr bool tl_allowed(int r) {
+  return r == 2 || r == 3 || r == 4 || r == 6 || r == 8 || r == 9 || r == 12 || r == 16;
+}
 __host__ __device__ constexpr int tl_nst(int n, int rmax) {
-  int s = 0;
-  for (int r = rmax; r >= 4; r /= 2)
-    while (n % r == 0) { n /= r; s++; }
-  while (n % 2 == 0) { n /= 2; s++; }
-  while (n % 3 == 0) { n /= 3; s++; }
-  return s;
+  if (n == 1) return 0;
+  int best = 99;
+  for (int r = 2; r <= rmax; r++)
+    if (tl_allowed(r) && n % r == 0) {
+      const int s = 1 + tl_nst(n / r, r);
+      if (s < best) best = s;
+    }
+  return best;
 }
 __host__ __device__ constexpr int tl_radix(int n, int idx, int rmax) {
-  int s = 0;
-  for (int r = rmax; r >= 4; r /= 2)
-    while (n % r == 0) { if (s == idx) return r; n /= r; s++; }
-  while (n % 2 == 0) { if (s == idx) return 2; n /= 2; s++; }
-  while (n % 3 == 0) { if (s == idx) return 3; n /= 3; s++; }
+  const int nst = tl_nst(n, rmax);
+  for (int s = 0; n > 1; s++) {
+    int r = 2;   // the smallest first radix from which the rest takes the remaining stages
+    while (!(tl_allowed(r) && n % r == 0 && tl_nst(n / r, r) == nst - 1 - s)) r++;
+    if (s == idx) return r;
+    n /= r;
+  }
   return 1;
 }
 
@@ -113,6 +121,53 @@ __device__ __forceinline__ void butterfly(c2<T>* v, int sign) {
     for (int k1 = 0; k1 < 4; k1++) {
       v[k1] = cadd<T>(e[k1], o[k1]);
       v[k1 + 4] = csub<T>(e[k1], o[k1]);
+    }
+  } else if constexpr (R == 6 || R == 12) {
+    // coprime factors Q (2 or 4) and 3: n = 3 n1 + Q n2 and the k with
+    // k = k1 (mod Q), k = k2 (mod 3) need no twiddles
+    constexpr int Q = R / 3;
+    c2<T> a[3][Q];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; n2++) {
+#pragma unroll
+      for (int n1 = 0; n1 < Q; n1++) a[n2][n1] = v[(3 * n1 + Q * n2) % R];
+      butterfly<T, Q>(a[n2], sign);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < Q; k1++) {
+      c2<T> b[3] = {a[0][k1], a[1][k1], a[2][k1]};
+      butterfly<T, 3>(b, sign);
+#pragma unroll
+      for (int k2 = 0; k2 < 3; k2++) v[((Q == 2 ? 3 : 9) * k1 + 4 * k2) % R] = b[k2];
+    }
+  } else if constexpr (R == 9) {
+    // n = n1 + 3 n2, k = k1 + 3 k2: DFT3 over n2, twiddle W9^(n1 k1), DFT3 over n1
+    constexpr double W9[3][2] = {{0.76604444311897803520, 0.64278760968653932632},
+                                 {0.17364817766693034885, 0.98480775301220805937},
+                                 {-0.93969262078590838405, 0.34202014332566873304}};   // W9^1, W9^2, W9^4
+    c2<T> a[3][3];
+#pragma unroll
+    for (int n1 = 0; n1 < 3; n1++) {
+      a[n1][0] = v[n1];
+      a[n1][1] = v[n1 + 3];
+      a[n1][2] = v[n1 + 6];
+      butterfly<T, 3>(a[n1], sign);
+    }
+    auto w9 = [&](c2<T> x, int m) {
+      const T c = (T)W9[m][0], s = (T)sign * (T)W9[m][1];
+      return mk<T>(x.x * c - x.y * s, x.x * s + x.y * c);
+    };
+    a[1][1] = w9(a[1][1], 0);
+    a[1][2] = w9(a[1][2], 1);
+    a[2][1] = w9(a[2][1], 1);
+    a[2][2] = w9(a[2][2], 2);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; k1++) {
+      c2<T> b[3] = {a[0][k1], a[1][k1], a[2][k1]};
+      butterfly<T, 3>(b, sign);
+      v[k1] = b[0];
+      v[k1 + 3] = b[1];
+      v[k1 + 6] = b[2];
     }
   } else if constexpr (R == 2) {
     c2<T> a = v[0], b = v[1];

@@ -105,10 +105,10 @@ void fill_float_consts(NewtonConst& nc);
 
 bool make_plan(int n, FftPlan* p);
 
-// TMA-staged passes (fft_tma.cu) for grids whose three line lengths have
-// compile-time plans.  tma_create builds the tensor maps over the fields and
+// TMA-staged passes (fft_tma.cuh) for line lengths with compile-time plans,
+// pass by pass (z: n2, strided: n0 and n1, x + Green: n0).  tma_create builds the tensor maps over the fields and
 // spectra; tma_has(t, pass) says whether pass 0 (z), 1 (y / x strided) or
-// 2 (x + Green) has them.  err: device flag raised by a timed-out wait.
+// 2 (x + Green) can run.  err: device flag raised by a timed-out wait.
 struct TmaMaps;
 template <typename T>
 TmaMaps* tma_create(const FftGeom& g, T* sig, T* strain, T* wspin, c2<T>* spec, c2<T>* anti, int ks = 0,
