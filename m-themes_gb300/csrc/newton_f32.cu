@@ -14,10 +14,10 @@ __device__ __noinline__ bool solve5_f64(const float* H, const float* b, float* x
 //
 // What bounds it: issue slots (0.70 of the cycles issue; the FP32 pipe is
 // half busy, DRAM a tenth).  128^3, 100 Green iterations, ms (events around
-// each launch): 37.5, against 103.5 for the earlier kernels, whose blocks
-// stepped their solves in lock step to share the FP64 solves; the FP32-solve
-// mode at 64^3 5.2 against 10.7, the dislocation-density law at 96^3 17.9
-// against 31.5.
+// each launch): 32.5, 37.4 with one system to an instruction, 103.5 for the
+// earlier kernels, whose blocks stepped their solves in lock step to share the
+// FP64 solves; the FP32-solve mode at 64^3 4.6, 5.2 and 10.7, the
+// dislocation-density law at 96^3 17.2, 17.9 and 31.5.
 template <int SOLVE, int LAW, bool GEN, int MINB>
 __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_constant__ LocalConst lc,
                                                                  Fields<float> f, double* __restrict__ partials,
@@ -95,8 +95,17 @@ __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_co
       float lam[6], u[6], R[9], ss[5], es[5];
 #pragma unroll
       for (int i = 0; i < 9; i++) R[i] = ld_again(f.rot + i * P + v);
-      dev_to_sample<float>(R, x, ss);
-      dev_to_sample<float>(R, ed, es);
+      {
+        float2 xe[5], se[5];
+#pragma unroll
+        for (int i = 0; i < 5; i++) xe[i] = make_float2(x[i], ed[i]);
+        dev_to_sample2(R, xe, se);
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+          ss[i] = se[i].x;
+          es[i] = se[i].y;
+        }
+      }
 #pragma unroll
       for (int i = 0; i < 6; i++) {
         lam[i] = ld_again(f.sig + i * P + v);
@@ -145,9 +154,8 @@ __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_co
 }
 
 // Blocks of 128 threads per SM the kernels are compiled for.  100 launches,
-// ms: 128^3 37.1 with 4 (128 registers, no spills), 38.8 with 5, 39.6 with 6
-// (80 registers, 280 B of spills); dislocation-density law at 96^3 17.5 with
-// 4, 19.3 with 3, 22.3 with 5.
+// ms: 128^3 33.3 with 4 (128 registers), 35.9 with 3, 36.1 with 5, 39.9 with 6;
+// dislocation-density law at 96^3 17.2 with 4, 19.0 with 3, 23.4 with 5.
 #ifndef MTH_F32_MINB
 #define MTH_F32_MINB 4
 #endif

@@ -243,7 +243,7 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
       {
         float H[15];
         Ldl5 f;
-        hessian_f32(pf, col, w, dt, H);
+        hessian_f32<LAW, GEN>(pf, col, w, dt, H);
         ok = ldl5_factor(H, f);
         ldl5_apply(f, rf, p);
       }
@@ -271,15 +271,12 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
       prev = step;
       if (done) {
         // rates at the accepted iterate: + sum_s w_s m_s (m_s . p)
+float2 g[NSYS / 2];
+        resolved2(pf, p, g);
+        const float sc = LAW == 0 ? pf.gn : 1.0f;
 #pragma unroll
-        for (int i = 0; i < 5; i++) edf[i] = 0;
-#pragma unroll
-        for (int s = 0; s < NSYS; s++) {
-          const float* m = pf.m[s];
-          const float g = w[s] * fmaf(m[4], p[4], fmaf(m[3], p[3], fmaf(m[2], p[2], fmaf(m[1], p[1], m[0] * p[0]))));
-#pragma unroll
-          for (int i = 0; i < 5; i++) edf[i] = fmaf(m[i], g, edf[i]);
-        }
+        for (int s = 0; s < NSYS; s++) at2(g[s / 2], s & 1) *= w[s] * sc;
+        rates2(pf, g, edf);
 #pragma unroll
         for (int i = 0; i < 5; i++) ed[i] += f32_to_f64(edf[i]);
       }
