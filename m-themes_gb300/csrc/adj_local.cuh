@@ -72,8 +72,9 @@ template <int K> ADJ_HD Dual<K> operator*(const Dual<K>& a, const Dual<K>& b) {
 }
 template <int K> ADJ_HD Dual<K> operator/(const Dual<K>& a, const Dual<K>& b) {
   Dual<K> r;
-  r.v = a.v / b.v;
-  for (int i = 0; i < K; i++) r.d[i] = (a.d[i] - r.v * b.d[i]) / b.v;
+  const double q = 1.0 / b.v;   // one division for the value and its derivatives
+  r.v = a.v * q;
+  for (int i = 0; i < K; i++) r.d[i] = (a.d[i] - r.v * b.d[i]) * q;
   return r;
 }
 template <int K> ADJ_HD Dual<K> operator*(double s, const Dual<K>& a) {
@@ -156,14 +157,15 @@ ADJ_HD void rot_increment(const N w[3], N C[3][3]) {
   N wt = dtan((0.5) * wn);
   if (fabs(val(wn)) < 1e-6) wn = num<N>(1.0);
   N ws[3];
-  for (int i = 0; i < 3; i++) ws[i] = w[i] * (wt / wn);
+  const N sc = wt / wn;
+  for (int i = 0; i < 3; i++) ws[i] = w[i] * sc;
   const N z = num<N>(0.0);
   N om[3][3] = {{z, (-1.0) * ws[2], ws[1]}, {ws[2], z, (-1.0) * ws[0]}, {(-1.0) * ws[1], ws[0], z}};
-  const N den = wt * wt + 1.0;
+  const N f = num<N>(2.0) / (wt * wt + 1.0);
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++) {
       N o2 = om[i][0] * om[0][j] + om[i][1] * om[1][j] + om[i][2] * om[2][j];
-      C[i][j] = (2.0) * ((om[i][j] + o2) / den) + (i == j ? 1.0 : 0.0);
+      C[i][j] = (om[i][j] + o2) * f + (i == j ? 1.0 : 0.0);
     }
 }
 
@@ -177,9 +179,27 @@ struct FlowEval {
   double ex[5], es[5];
 };
 
+// a^e for a > 0; whole and half e up to 63 by repeated squaring (12 calls of
+// pow are about 1500 of the FP64 operations a voxel has)
+ADJ_HD double pow_rate(double a, double e) {
+  const int k = e >= 1.0 && e < 64.0 ? (int)e : 0;
+  const double rest = e - (double)k;
+  if (k == 0 || (rest != 0.0 && rest != 0.5)) return pow(a, e);
+  double p = rest != 0.0 ? sqrt(a) : 1.0;
+  for (int b = k;;) {
+    if (b & 1) p *= a;
+    if (!(b >>= 1)) return p;
+    a *= a;
+  }
+}
+
 ADJ_HD void flow_eval(const PhaseConst& ph, const double sig[6], const double R[9], const double* tau, int flow_off,
                       FlowEval& f) {
-  rot_to_q<double>(R, f.Q);
+  {
+    double r9[9];
+    for (int i = 0; i < 9; i++) r9[i] = R[i];
+    rot_to_q_dev<double>(r9, f.Q);
+  }
   for (int i = 0; i < 5; i++) {
     double a = 0;
     for (int j = 0; j < 5; j++) a += f.Q[i * 5 + j] * sig[j];
@@ -193,13 +213,13 @@ ADJ_HD void flow_eval(const PhaseConst& ph, const double sig[6], const double R[
     double rss = 0;
     for (int i = 0; i < 5; i++) rss += ph.m_xt[s][i] * f.x[i];
     const double tp = rss < 0.0 ? tau[s] + ph.tau_back_minus_fwd : tau[s];
-    const double r = rss / tp, ar = fabs(r);
-    const double pnm1 = ar > 0.0 ? pow(ar, n - 1.0) : 0.0;
+    const double it = 1.0 / tp, r = rss * it, ar = fabs(r);
+    const double pnm1 = ar > 0.0 ? pow_rate(ar, n - 1.0) : 0.0;
     const double pn = pnm1 * ar;
     const double g = g0 * (r > 0.0 ? pn : -pn);
     f.gdot[s] = g;
-    f.w[s] = g0 * n * pnm1 / tp;
-    f.dgdtau[s] = -n * g / tp;
+    f.w[s] = g0 * n * pnm1 * it;
+    f.dgdtau[s] = -n * g * it;
     f.dgdn[s] = ar > 0.0 ? g * log(ar) : 0.0;
     for (int i = 0; i < 5; i++) f.ex[i] += ph.m_xt[s][i] * g;
   }
@@ -334,15 +354,12 @@ ADJ_HD void adj_pre(const PhaseConst& ph, const StepFlags& sf, const double sig[
                                           dvar<5>(ph.thet0, 3), dvar<5>(ph.thet1, 4), 1e-4 * ph.tau0f);
       const double F = V.v / dgam;
       double A = 0;   // sum_s taubar'_s a_s,  a_s = dt sum_j h_sj |gdot_j|
-      double hb[NSYS];
-      for (int j = 0; j < NSYS; j++) hb[j] = 0.0;
-      for (int s = 0; s < ph.nsys; s++) {
+      double hb[NSYS];   // taubar' h, so that A = dt sum_j hb_j |gdot_j|
+      for (int j = 0; j < ph.nsys; j++) {
         double a = 0;
-        for (int j = 0; j < ph.nsys; j++) {
-          a += ph.hard[s][j] * fabs(f.gdot[j]) * dt;
-          hb[j] += in.tau[s] * ph.hard[s][j];
-        }
-        A += in.tau[s] * a;
+        for (int s = 0; s < ph.nsys; s++) a += in.tau[s] * ph.hard[s][j];
+        hb[j] = a;
+        A += a * (fabs(f.gdot[j]) * dt);
       }
       const double dgbar = A * (V.d[1] - F) / dgam + in.gam;
       out.gam += A * V.d[0] / dgam;
@@ -379,7 +396,8 @@ ADJ_HD void adj_pre(const PhaseConst& ph, const StepFlags& sf, const double sig[
   for (int i = 0; i < 6; i++) sigbar[i] = seed6[i];
   double xb[5] = {0, 0, 0, 0, 0};
   for (int s = 0; s < ph.nsys; s++) {
-    for (int i = 0; i < 5; i++) xb[i] += gbar[s] * f.w[s] * ph.m_xt[s][i];
+    const double gw = gbar[s] * f.w[s];
+    for (int i = 0; i < 5; i++) xb[i] += gw * ph.m_xt[s][i];
     out.tau[s] += gbar[s] * f.dgdtau[s];
     th[3] += gbar[s] * f.dgdn[s];
   }
@@ -416,7 +434,8 @@ ADJ_HD void adj_post(const PhaseConst& ph, const StepFlags& sf, const double sig
   for (int s = 0; s < ph.nsys; s++) {
     double gb = 0;
     for (int i = 0; i < 5; i++) gb += ph.m_xt[s][i] * ebx[i];
-    for (int i = 0; i < 5; i++) xb[i] += gb * f.w[s] * ph.m_xt[s][i];
+    const double gw = gb * f.w[s];
+    for (int i = 0; i < 5; i++) xb[i] += gw * ph.m_xt[s][i];
     st.tau[s] += gb * f.dgdtau[s];
     th[3] += gb * f.dgdn[s];
   }
@@ -445,8 +464,10 @@ ADJ_HD bool tangent_stiffness(const PhaseConst& ph, const StepFlags& sf, const F
   for (int i = 0; i < 15; i++) Dx[i] = 0.0;
   if (!sf.flow_off)
     for (int s = 0; s < ph.nsys; s++)
-      for (int i = 0; i < 5; i++)
-        for (int j = i; j < 5; j++) Dx[pk5(i, j)] += f.w[s] * ph.m_xt[s][i] * ph.m_xt[s][j];
+      for (int i = 0; i < 5; i++) {
+        const double wm = f.w[s] * ph.m_xt[s][i];
+        for (int j = i; j < 5; j++) Dx[pk5(i, j)] += wm * ph.m_xt[s][j];
+      }
   // M = S + dt Q^T Dx Q
   double M[5][5], T[5][5];
   for (int i = 0; i < 5; i++)
@@ -456,35 +477,35 @@ ADJ_HD bool tangent_stiffness(const PhaseConst& ph, const StepFlags& sf, const F
       T[i][j] = a;
     }
   for (int i = 0; i < 5; i++)
-    for (int j = 0; j < 5; j++) {
+    for (int j = 0; j <= i; j++) {
       double a = 0;
       for (int k = 0; k < 5; k++) a += f.Q[k * 5 + i] * T[k][j];
       M[i][j] = sel[pk5(i, j)] + sf.dt * a;
     }
-  // LDL^T of M, then the inverse column by column
-  double L[5][5], d[5];
+  // LDL^T of M (lower triangle), then the inverse column by column
+  double L[5][5], d[5], id[5];
   for (int j = 0; j < 5; j++) {
     double dj = M[j][j];
     for (int k = 0; k < j; k++) dj -= L[j][k] * L[j][k] * d[k];
     if (!(dj > 0.0)) return false;
     d[j] = dj;
-    L[j][j] = 1.0;
+    id[j] = 1.0 / dj;
     for (int i = j + 1; i < 5; i++) {
       double a = M[i][j];
       for (int k = 0; k < j; k++) a -= L[i][k] * L[j][k] * d[k];
-      L[i][j] = a / dj;
+      L[i][j] = a * id[j];
     }
   }
   double Ci[5][5];
   for (int c = 0; c < 5; c++) {
     double y[5];
     for (int i = 0; i < 5; i++) {
-      double a = (i == c) ? 1.0 : 0.0;
-      for (int k = 0; k < i; k++) a -= L[i][k] * y[k];
+      double a = (i == c) ? 1.0 : 0.0;   // y[i] = 0 above c
+      for (int k = c; k < i; k++) a -= L[i][k] * y[k];
       y[i] = a;
     }
     for (int i = 4; i >= 0; i--) {
-      double a = y[i] / d[i];
+      double a = i < c ? 0.0 : y[i] * id[i];
       for (int k = i + 1; k < 5; k++) a -= L[k][i] * Ci[k][c];
       Ci[i][c] = a;
     }
