@@ -166,21 +166,78 @@ __global__ void __launch_bounds__(256) adj_sum_tau_kernel(const double* __restri
 }
 
 // ------------------------------------------------------------ CG kernels
-// update_p: p = r + beta p first; then out = C_t p.
+// The sums of one iteration end on the device: each block leaves its partial
+// sum, the last one to finish adds them in a fixed order and does the scalar
+// step, so a solve's iterations need no host round trip.
+
+// v summed over the grid; true for thread 0 of the last block, with the total
+__device__ __forceinline__ bool adj_grid_sum(double v, double* __restrict__ partials, unsigned* ticket, double& total) {
+  constexpr int NT = 256;
+  __shared__ double sv[NT / 32];
+  __shared__ bool last;
+  const int t = threadIdx.x;
+  auto block = [&](double x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((t & 31) == 0) sv[t >> 5] = x;
+    __syncthreads();
+    double a = 0.0;
+    if (t == 0)
+      for (int k = 0; k < NT / 32; k++) a += sv[k];
+    return a;
+  };
+  const double a = block(v);
+  if (t == 0) {
+    __stcg(&partials[blockIdx.x], a);
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  double s = 0.0;
+  for (unsigned i = t; i < gridDim.x; i += NT) s += __ldcg(&partials[i]);
+  __syncthreads();
+  total = block(s);
+  if (t == 0) *ticket = 0;
+  return t == 0;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) adj_cg_start_kernel(const T* __restrict__ r, long long P, double tol, int itmax,
+                                                           AdjCg* __restrict__ cg, double* __restrict__ partials) {
+  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  double s = 0.0, rr;
+  if (v < P)
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+      const double x = to_f64(r[i * P + v]);
+      s += x * x;
+    }
+  if (!adj_grid_sum(s, partials, &cg->ticket, rr)) return;
+  cg->rr = rr;
+  cg->stop = tol * tol * rr;
+  cg->alpha = cg->beta = cg->pap = 0.0;
+  cg->it = cg->status = 0;
+  cg->itmax = itmax;
+  cg->live = rr > 0.0 && itmax > 0;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) adj_ct_apply_kernel(const T* __restrict__ ct, T* __restrict__ p,
-                                                           const T* __restrict__ r, T beta, int update_p,
-                                                           T* __restrict__ out, long long P) {
+                                                           const T* __restrict__ r, T* __restrict__ out, long long P,
+                                                           const AdjCg* __restrict__ cg) {
+  if (!cg->live) return;
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= P) return;
+  const bool first = cg->it == 0;
+  const T beta = (T)cg->beta;
   T x[6], c[16], y[6];
 #pragma unroll
   for (int i = 0; i < 6; i++) {
-    T pv = p[i * P + v];
-    if (update_p) {
-      pv = r[i * P + v] + beta * pv;
-      p[i * P + v] = pv;
-    }
+    T pv = r[i * P + v];
+    if (!first) pv += beta * p[i * P + v];
+    p[i * P + v] = pv;
     x[i] = pv;
   }
 #pragma unroll
@@ -191,23 +248,32 @@ __global__ void __launch_bounds__(256) adj_ct_apply_kernel(const T* __restrict__
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) adj_dot_kernel(const T* __restrict__ a, const T* __restrict__ b, long long P,
-                                                      double* __restrict__ partials) {
+__global__ void __launch_bounds__(256) adj_cg_dot_kernel(const T* __restrict__ a, const T* __restrict__ b, long long P,
+                                                         AdjCg* __restrict__ cg, double* __restrict__ partials) {
+  if (!cg->live) return;
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double s[1] = {0.0};
+  double s = 0.0, pap;
   if (v < P)
 #pragma unroll
-    for (int i = 0; i < 6; i++) s[0] += to_f64(a[i * P + v]) * to_f64(b[i * P + v]);   // exact products
-  adj_block_sum<1>(s, partials);
+    for (int i = 0; i < 6; i++) s += to_f64(a[i * P + v]) * to_f64(b[i * P + v]);   // exact products
+  if (!adj_grid_sum(s, partials, &cg->ticket, pap)) return;
+  cg->pap = pap;
+  if (pap > 0.0) cg->alpha = cg->rr / pap;
+  else {
+    cg->status = 1;
+    cg->live = 0;
+  }
 }
 
-// x += alpha p ; r -= alpha Ap ; partial |r|^2
+// x += alpha p ; r -= alpha Ap ; |r|^2
 template <typename T>
 __global__ void __launch_bounds__(256) adj_cg_update_kernel(T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
-                                                            const T* __restrict__ ap, T alpha, long long P,
-                                                            double* __restrict__ partials) {
+                                                            const T* __restrict__ ap, long long P,
+                                                            AdjCg* __restrict__ cg, double* __restrict__ partials) {
+  if (!cg->live) return;
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double s[1] = {0.0};
+  const T alpha = (T)cg->alpha;
+  double s = 0.0, rn;
   if (v < P)
 #pragma unroll
     for (int i = 0; i < 6; i++) {
@@ -215,9 +281,19 @@ __global__ void __launch_bounds__(256) adj_cg_update_kernel(T* __restrict__ x, T
       x[o] += alpha * p[o];
       const T rv = r[o] - alpha * ap[o];
       r[o] = rv;
-      s[0] += to_f64(rv) * to_f64(rv);
+      s += to_f64(rv) * to_f64(rv);
     }
-  adj_block_sum<1>(s, partials);
+  if (!adj_grid_sum(s, partials, &cg->ticket, rn)) return;
+  cg->it++;
+  if (!isfinite(rn)) {
+    cg->status = 2;
+    cg->live = 0;
+  } else if (rn <= cg->stop || cg->it >= cg->itmax) {
+    cg->live = 0;
+  } else {
+    cg->beta = rn / cg->rr;
+    cg->rr = rn;
+  }
 }
 
 // --------------------------------------------------- Fourier projection
@@ -325,7 +401,8 @@ template <typename T, int NC>
 __global__ void __launch_bounds__(256) adj_x_proj_kernel(const AdjProj pj, c2<T>* __restrict__ spec, int nin,
                                                          long long kplane, int n0_, int n1, int n2, int kzn, int kzs,
                                                          int kb, FftPlan pl, const c2<T>* __restrict__ twf,
-                                                         const c2<T>* __restrict__ twi) {
+                                                         const c2<T>* __restrict__ twi, const int* __restrict__ live) {
+  if (live && !*live) return;
   const int n0 = NC > 0 ? NC : n0_;
   extern __shared__ unsigned char smraw[];
   c2<T>* tw_f = reinterpret_cast<c2<T>*>(smraw);
@@ -390,26 +467,31 @@ cudaError_t launch_adj_sum_tau(const double* tau, int nsys, long long P, double*
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t launch_adj_ct_apply(const T* ct, T* p, const T* r, double beta, int update_p, T* out, long long P,
+cudaError_t launch_adj_cg_start(const T* r, long long P, double tol, int itmax, AdjCg* cg, double* partials,
                                 cudaStream_t st) {
-  adj_ct_apply_kernel<T><<<blocks_of(P), 256, 0, st>>>(ct, p, r, (T)beta, update_p, out, P);
+  adj_cg_start_kernel<T><<<blocks_of(P), 256, 0, st>>>(r, P, tol, itmax, cg, partials);
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t launch_adj_dot(const T* a, const T* b, long long P, double* partials, cudaStream_t st) {
-  adj_dot_kernel<T><<<blocks_of(P), 256, 0, st>>>(a, b, P, partials);
+cudaError_t launch_adj_ct_apply(const T* ct, T* p, const T* r, T* out, long long P, const AdjCg* cg, cudaStream_t st) {
+  adj_ct_apply_kernel<T><<<blocks_of(P), 256, 0, st>>>(ct, p, r, out, P, cg);
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t launch_adj_cg_update(T* x, T* r, const T* p, const T* ap, double alpha, long long P, double* partials,
+cudaError_t launch_adj_cg_dot(const T* p, const T* ap, long long P, AdjCg* cg, double* partials, cudaStream_t st) {
+  adj_cg_dot_kernel<T><<<blocks_of(P), 256, 0, st>>>(p, ap, P, cg, partials);
+  return cudaGetLastError();
+}
+template <typename T>
+cudaError_t launch_adj_cg_update(T* x, T* r, const T* p, const T* ap, long long P, AdjCg* cg, double* partials,
                                  cudaStream_t st) {
-  adj_cg_update_kernel<T><<<blocks_of(P), 256, 0, st>>>(x, r, p, ap, (T)alpha, P, partials);
+  adj_cg_update_kernel<T><<<blocks_of(P), 256, 0, st>>>(x, r, p, ap, P, cg, partials);
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_adj_x_proj(const FftGeom& g, const AdjProj& pj, c2<T>* spec, int nin, const c2<T>* twf,
-                              const c2<T>* twi, cudaStream_t st) {
+                              const c2<T>* twi, const int* live, cudaStream_t st) {
   int kb = 16;
   auto smem = [&](int kbv) { return sizeof(c2<T>) * ((size_t)2 * g.n0 + 2 * (size_t)nin * kbv * (g.n0 + 1)); };
   while (kb > 1 && smem(kb) > g.smem_budget) kb >>= 1;
@@ -423,7 +505,7 @@ cudaError_t launch_adj_x_proj(const FftGeom& g, const AdjProj& pj, c2<T>* spec, 
   }
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   dim3 grid((g.kz + kb - 1) / kb, g.n1);
-  k<<<grid, 256, sm, st>>>(pj, spec, nin, g.kplane, g.n0, g.n1, g.n2, g.kz, g.kzs, kb, g.px, twf, twi);
+  k<<<grid, 256, sm, st>>>(pj, spec, nin, g.kplane, g.n0, g.n1, g.n2, g.kz, g.kzs, kb, g.px, twf, twi, live);
   return cudaGetLastError();
 }
 
@@ -432,12 +514,13 @@ cudaError_t launch_adj_x_proj(const FftGeom& g, const AdjProj& pj, c2<T>* spec, 
                                          const double*, double*, cudaStream_t);                                    \
   template cudaError_t launch_adj_post<T>(const NewtonConst&, const AdjStepArgs&, const AdjViews<T>&, double*,    \
                                           cudaStream_t);                                                           \
-  template cudaError_t launch_adj_ct_apply<T>(const T*, T*, const T*, double, int, T*, long long, cudaStream_t); \
-  template cudaError_t launch_adj_dot<T>(const T*, const T*, long long, double*, cudaStream_t);                   \
-  template cudaError_t launch_adj_cg_update<T>(T*, T*, const T*, const T*, double, long long, double*,            \
+  template cudaError_t launch_adj_cg_start<T>(const T*, long long, double, int, AdjCg*, double*, cudaStream_t);   \
+  template cudaError_t launch_adj_ct_apply<T>(const T*, T*, const T*, T*, long long, const AdjCg*, cudaStream_t); \
+  template cudaError_t launch_adj_cg_dot<T>(const T*, const T*, long long, AdjCg*, double*, cudaStream_t);        \
+  template cudaError_t launch_adj_cg_update<T>(T*, T*, const T*, const T*, long long, AdjCg*, double*,            \
                                                cudaStream_t);                                                      \
   template cudaError_t launch_adj_x_proj<T>(const FftGeom&, const AdjProj&, c2<T>*, int, const c2<T>*,          \
-                                            const c2<T>*, cudaStream_t);
+                                            const c2<T>*, const int*, cudaStream_t);
 INST(float)
 INST(double)
 #undef INST

@@ -43,8 +43,11 @@ struct AdjRun {
   char* p = nullptr;
   char* ap = nullptr;
   char* tmp = nullptr;
+  AdjCg* cg = nullptr;
+  TmaMaps* tma = nullptr;   // tile passes from tmp over spec9 to ap
   std::vector<HostCkpt> hck;
   ~AdjRun() {
+    tma_destroy(tma);
     for (void* m : mem) cudaFree(m);
   }
   cudaError_t alloc(void** out, size_t bytes) {
@@ -130,23 +133,37 @@ static mth_status adj_forward_step(mth_ctx* c, AdjRun& run, int slot, double* s3
 // out = Q(in) (nin = 6) or Q(in[0..5]) + W^T(in[6..8]) (nin = 9): the
 // forward's z and y passes around the projection x pass
 template <typename T>
-static cudaError_t adj_project_launch(mth_ctx* c, AdjRun& run, const AdjProj& pj, const T* in, int nin, T* out) {
+static cudaError_t adj_project_launch(mth_ctx* c, AdjRun& run, const AdjProj& pj, const T* in, int nin, T* out,
+                                      const int* live) {
   const FftGeom& g = c->geom;
   c2<T>* sp = reinterpret_cast<c2<T>*>(run.spec9);
   auto tw = [&](int a, int d) { return static_cast<const c2<T>*>(c->tw[a][d]); };
-  const IterIn none{nullptr, nullptr};
-  cudaError_t e = launch_fft_z_r2c<T>(g, in, sp, nin, tw(2, 0), none, c->st);
-  if (e == cudaSuccess) e = launch_fft_strided<T>(g, sp, nin, 1, -1, tw(1, 0), none, c->st);
-  if (e == cudaSuccess) e = launch_adj_x_proj<T>(g, pj, sp, nin, tw(0, 0), tw(0, 1), c->st);
-  if (e == cudaSuccess) e = launch_fft_strided<T>(g, sp, 6, 1, +1, tw(1, 1), none, c->st);
-  if (e == cudaSuccess) e = launch_fft_z_c2r<T>(g, sp, out, 6, tw(2, 1), (T)(1.0 / (double)c->nv), none, 0, c->st);
+  const IterIn it{nullptr, live, 0};
+  const T scale = (T)(1.0 / (double)c->nv);
+  // the solve's projections (tmp -> ap) by the tile passes, as the forward's
+  // (187 iterations at 64^3, FP32: their kernels 21.9 against 29.0 ms)
+  const bool tile = in == reinterpret_cast<const T*>(run.tmp) && out == reinterpret_cast<T*>(run.ap) && nin == 6;
+  const bool tz = tile && tma_has(run.tma, 0), ts = tile && tma_has(run.tma, 1);
+  cudaError_t e = tz ? tma_fft_z_r2c<T>(run.tma, g, tw(2, 0), it, c->err_d, c->st)
+                     : launch_fft_z_r2c<T>(g, in, sp, nin, tw(2, 0), it, c->st);
+  if (e == cudaSuccess)
+    e = ts ? tma_fft_strided<T>(run.tma, g, 0, -1, tw(1, 0), it, c->err_d, c->st)
+           : launch_fft_strided<T>(g, sp, nin, 1, -1, tw(1, 0), it, c->st);
+  if (e == cudaSuccess) e = launch_adj_x_proj<T>(g, pj, sp, nin, tw(0, 0), tw(0, 1), live, c->st);
+  if (e == cudaSuccess)
+    e = ts ? tma_fft_strided<T>(run.tma, g, 0, +1, tw(1, 1), it, c->err_d, c->st)
+           : launch_fft_strided<T>(g, sp, 6, 1, +1, tw(1, 1), it, c->st);
+  if (e == cudaSuccess)
+    e = tz ? tma_fft_z_c2r<T>(run.tma, g, 2, tw(2, 1), scale, it, c->err_d, c->st)
+           : launch_fft_z_c2r<T>(g, sp, out, 6, tw(2, 1), scale, it, 0, c->st);
   return e;
 }
 template <typename T>
-static mth_status adj_project(mth_ctx* c, AdjRun& run, const AdjProj& pj, const T* in, int nin, T* out) {
+static mth_status adj_project(mth_ctx* c, AdjRun& run, const AdjProj& pj, const T* in, int nin, T* out,
+                              const int* live = nullptr) {
   const FftGeom& g = c->geom;
   const double w = sizeof(T), rp = w * (double)c->nv, kp = 2.0 * w * (double)g.n0 * g.n1 * g.kz;
-  LAUNCHN(K_ADJ_CG, 5, (nin + 6) * (rp + 2 * kp) + 2 * nin * kp, adj_project_launch<T>(c, run, pj, in, nin, out));
+  LAUNCHN(K_ADJ_CG, 5, (nin + 6) * (rp + 2 * kp) + 2 * nin * kp, adj_project_launch<T>(c, run, pj, in, nin, out, live));
   return MTH_OK;
 }
 
@@ -201,40 +218,38 @@ static mth_status adj_reverse_step(mth_ctx* c, AdjRun& run, int step, int slot, 
   s = adj_project<T>(c, run, pj, reinterpret_cast<const T*>(run.rhs), 9, r);
   if (s) return s;
   CK(cudaMemsetAsync(mu, 0, b6, c->st));
-  LAUNCH(K_ADJ_CG, 12.0 * w * P, launch_adj_dot<T>(r, r, P, c->partials, c->st));
-  double rr0;
-  s = reduce_to_host(c, 1, &rr0);
-  if (s) return s;
-  int it = 0;
-  if (rr0 > 0.0) {
-    CK(cudaMemcpyAsync(p, r, b6, cudaMemcpyDeviceToDevice, c->st));
-    double rr = rr0, beta = 0.0;
-    const double stop = tol * tol * rr0;
-    for (; it < itmax;) {
-      LAUNCH(K_ADJ_CG, (it ? 18.0 : 12.0) * w * P + 16.0 * w * P,
-             launch_adj_ct_apply<T>(ct, p, r, beta, it > 0, tmp, P, c->st));
-      s = adj_project<T>(c, run, pj, tmp, 6, ap);
+  AdjCg* cg = run.cg;
+  LAUNCH(K_ADJ_CG, 6.0 * w * P, launch_adj_cg_start<T>(r, P, tol, itmax, cg, c->partials, c->st));
+  // iterations are queued CG_AHEAD at a time; the kernels of those past the
+  // end return at once (64^3, 187 iterations in 4 solves: 88.7 ms for the
+  // whole gradient, 102.2 ms with two host round trips an iteration and the
+  // shared-memory passes)
+  constexpr int CG_AHEAD = 8;
+  AdjCg h;
+  static_assert(sizeof(AdjCg) <= sizeof(double) * NPART, "read back through the sums' pinned buffer");
+  for (int queued = 0;;) {
+    for (int k = 0; k < CG_AHEAD && queued < itmax; k++, queued++) {
+      LAUNCH(K_ADJ_CG, (queued ? 18.0 : 12.0) * w * P + 16.0 * w * P,
+             launch_adj_ct_apply<T>(ct, p, r, tmp, P, cg, c->st));
+      s = adj_project<T>(c, run, pj, tmp, 6, ap, &cg->live);
       if (s) return s;
-      LAUNCH(K_ADJ_CG, 12.0 * w * P, launch_adj_dot<T>(p, ap, P, c->partials, c->st));
-      double pap;
-      s = reduce_to_host(c, 1, &pap);
-      if (s) return s;
-      if (!(pap > 0.0))
-        return set_err(MTH_ERR_NAN, "adjoint: projected tangent operator not positive (step %d, p.Ap=%g)", step, pap);
-      const double alpha = rr / pap;
-      LAUNCH(K_ADJ_CG, 36.0 * w * P, launch_adj_cg_update<T>(mu, r, p, ap, alpha, P, c->partials, c->st));
-      double rn;
-      s = reduce_to_host(c, 1, &rn);
-      if (s) return s;
-      it++;
-      if (!std::isfinite(rn)) return set_err(MTH_ERR_NAN, "adjoint: non-finite CG residual");
-      if (rn <= stop) break;
-      beta = rn / rr;
-      rr = rn;
+      LAUNCH(K_ADJ_CG, 12.0 * w * P, launch_adj_cg_dot<T>(p, ap, P, cg, c->partials, c->st));
+      LAUNCH(K_ADJ_CG, 36.0 * w * P, launch_adj_cg_update<T>(mu, r, p, ap, P, cg, c->partials, c->st));
     }
-    if (it >= itmax)
-      return set_err(MTH_ERR_NOT_CONVERGED, "adjoint: CG did not reach %g in %d iterations (step %d)", tol, itmax, step);
+    CK(cudaMemcpyAsync(c->red_h, cg, sizeof(AdjCg), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(c->err_h, c->err_d, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    prof_resolve(c);
+    if (*c->err_h) return set_err(MTH_ERR_TIMEOUT, "a kernel timed out waiting for its tile copies");
+    memcpy(&h, c->red_h, sizeof(h));
+    if (!h.live) break;
   }
+  const int it = h.it;
+  if (h.status == 1)
+    return set_err(MTH_ERR_NAN, "adjoint: projected tangent operator not positive (step %d, p.Ap=%g)", step, h.pap);
+  if (h.status == 2) return set_err(MTH_ERR_NAN, "adjoint: non-finite CG residual");
+  if (it >= itmax)
+    return set_err(MTH_ERR_NOT_CONVERGED, "adjoint: CG did not reach %g in %d iterations (step %d)", tol, itmax, step);
   *iters = it;
   LAUNCH(K_ADJ_LOCAL, (double)P * (31 * w + 22 * 8 * 2 + 6 * 8 + 22 * w),
          launch_adj_post<T>(c->nc, a, v, c->partials, c->st));
@@ -288,6 +303,12 @@ extern "C" mth_status mth_adjoint(mth_ctx* c, const mth_adjoint_opts* o, double*
   CK(run.alloc(&m, 6 * pl)); run.p = (char*)m;
   CK(run.alloc(&m, 6 * pl)); run.ap = (char*)m;
   CK(run.alloc(&m, 6 * pl)); run.tmp = (char*)m;
+  CK(run.alloc(&m, sizeof(AdjCg))); run.cg = (AdjCg*)m;
+  CK(cudaMemsetAsync(run.cg, 0, sizeof(AdjCg), c->st));
+  run.tma = c->mixed ? tma_create<float>(c->geom, (float*)run.tmp, (float*)run.ap, (float*)run.ap,
+                                         (c2<float>*)run.spec9, (c2<float>*)run.spec9)
+                     : tma_create<double>(c->geom, (double*)run.tmp, (double*)run.ap, (double*)run.ap,
+                                          (c2<double>*)run.spec9, (c2<double>*)run.spec9);
   run.hck.resize(nseg + 1);
   // k = 0 block of the projection: stress-controlled diagonal components
   AdjProj pj;

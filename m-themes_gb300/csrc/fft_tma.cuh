@@ -234,15 +234,15 @@ __host__ __device__ constexpr int rmax_tile(int L, int lines) {
 
 // Threads per block of a tile of `lines` lines of L points under radix cap
 // rmax: the multiple of 32 from lo to 384 that leaves the fewest threads idle
-// over the plan's stages and a pass over `extra` further points (256, if it is
+// over the plan's stages and passes over `extra` and `extra2` further points (256, if it is
 // one of the best).  The strided and Green passes (lo 128) are all stages:
 // 128^3 FP32 y 41.2 / 45.2 us with 128 / 256 threads, x + Green 43.2 / 47.0 us
 // with 192 / 256.  The z passes (lo 192) also split or merge: C2R of 128^3 33.1 /
 // 35.1 us with 256 / 192, of 96^3 18.8 / 20.5 us with 192 / 256.
-__host__ __device__ constexpr int nt_tile(int L, int lines, int rmax, int lo = 128, int extra = 0) {
+__host__ __device__ constexpr int nt_tile(int L, int lines, int rmax, int lo = 128, int extra = 0, int extra2 = 0) {
   int best = 256, cost = 1 << 30;
   for (int nt = 384; nt >= lo; nt -= 32) {
-    int c = (extra + nt - 1) / nt * nt;
+    int c = (extra + nt - 1) / nt * nt + (extra2 + nt - 1) / nt * nt;
     for (int s = 0; s < tl_nst(L, rmax); s++) {
       const int t = L / tl_radix(L, s, rmax) * lines;
       c += (t + nt - 1) / nt * nt;
@@ -285,7 +285,7 @@ template <typename T> __host__ __device__ constexpr int lb_z(int n, int elems) {
 __host__ __device__ constexpr int nt_zr(int n, int lb) {
   return nt_tile(n / 2, lb, RMAX_Z, 192, lb * ((n / 2 + 2) & ~1));
 }
-__host__ __device__ constexpr int nt_zc(int n, int lb) { return nt_tile(n / 2, lb, RMAX_Z, 192, lb * n * 3 / 2); }
+__host__ __device__ constexpr int nt_zc(int n, int lb) { return nt_tile(n / 2, lb, RMAX_Z, 192, lb * n / 2, lb * n); }
 // r2c: one block = LB consecutive (x,y) lines of one stress component.
 template <typename T, int N, int LB>
 __global__ void __launch_bounds__(nt_zr(N, LB)) fft_zr_tma_kernel(
@@ -691,15 +691,15 @@ cudaError_t tma_fft_z_r2c(const TmaMaps* t, const FftGeom& g, const c2<T>* tw, c
   }
 }
 
-// which = 0: stress spectrum -> strain field (mode 1); 1: spin spectrum ->
-// spin field (mode 0)
+// which = 0: stress spectrum added to the strain field; 1: spin spectrum ->
+// spin field; 2: stress spectrum -> strain field
 template <typename T>
 cudaError_t tma_fft_z_c2r(const TmaMaps* t, const FftGeom& g, int which, const c2<T>* tw, T scale, const IterIn& it,
                           int* err, cudaStream_t st) {
   const long long lines = (long long)g.n0 * g.n1;
-  const c2<T>* ms = static_cast<const c2<T>*>(which ? t->anti : t->spec);
-  T* mr = static_cast<T*>(which ? t->wspin : t->strain);
-  const int ncomp = which ? 3 : 6, mode = which ? 0 : 1;
+  const c2<T>* ms = static_cast<const c2<T>*>(which == 1 ? t->anti : t->spec);
+  T* mr = static_cast<T*>(which == 1 ? t->wspin : t->strain);
+  const int ncomp = which == 1 ? 3 : 6, mode = which == 0;
   switch (g.n2) {
 #define MTH_CASE(N) case N: return zc_launch<T, N>(ms, mr, ncomp, lines, tw, scale, it, mode, err, st);
     MTH_TMA_SIZES(MTH_CASE)
