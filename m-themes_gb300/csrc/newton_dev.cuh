@@ -786,7 +786,11 @@ inline void fill_local(const NewtonConst& nc, bool predictor, LocalConst& lc) {
     s.chord2 = ph.type == 0 ? (float)pow(0.4 * nc.tol / (ph.nrs * ph.nrs), 2.0 / 3.0) : 0.0f;   // n^2 d^3 / 2 <= tol / 5
     for (int i = 0; i < NSYS; i++) {
       int q = 0;
-      for (int a = 0; a < 5; a++) (i & 1 ? s.m[i / 2][a].y : s.m[i / 2][a].x) = (float)ph.m_xt[i][a];
+      for (int a = 0; a < 5; a++) {
+        const float hi = (float)ph.m_xt[i][a], lo = (float)(ph.m_xt[i][a] - (double)hi);
+        (i & 1 ? s.m[i / 2][a].y : s.m[i / 2][a].x) = hi;
+        (i & 1 ? s.ml[i / 2][a].y : s.ml[i / 2][a].x) = lo;
+      }
       for (int a = 0; a < 5; a++)
         for (int b = a; b < 5; b++, q++)
           (q & 1 ? s.mm[i][q / 2].y : s.mm[i][q / 2].x) = (float)(ph.m_xt[i][a] * ph.m_xt[i][b]);

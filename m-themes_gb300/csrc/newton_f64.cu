@@ -21,10 +21,10 @@ namespace mth {
 // the step squared).  A start that fails, a step above 1e-2 |lambda|, or no
 // end within eight steps falls back to the damped FP64 iteration from
 // lambda (solve_full), which tight iteration caps use from the start.
-// What bounds it is still the FP64 pipe (0.85 busy), with 1150 FP64 warp
-// instructions a solve instead of about 6700: 128^3, 4.0 ms per launch
+// What bounds it is still the FP64 pipe, with about 800 FP64 warp
+// instructions a solve instead of about 6700: 128^3, 3.5 ms per launch
 // against 24.0 with every pass in FP64, the same fields to 1e-15; the array
-// solve of 100 003 points 0.34 against 4.2 ms.
+// solve of 100 003 points 0.31 against 4.2 ms.
 
 // what the fallback reads and returns
 struct FullIo {
@@ -110,6 +110,87 @@ __device__ __forceinline__ void rates_f64(const PhaseConst& ph, const SlipF& pf,
       }
     }
   }
+}
+
+// A number as the unevaluated sum h + l of two FP32 numbers, two at a time
+struct F2x2 {
+  float2 h, l;
+};
+// (s, c) += (a + al) (b + bl): the rounding errors of the leading product and of
+// the sum are kept in c
+__device__ __forceinline__ void acc2(F2x2& s, float2 a, float2 al, float2 b, float2 bl) {
+  const float2 m1 = make_float2(-1.0f, -1.0f);
+  const float2 p = mul2(a, b), t = add2(s.h, p), z = fma2(s.h, m1, t);
+  float2 e = fma2(a, b, mul2(p, m1));   // a b - p
+  e = fma2(a, bl, e);
+  e = fma2(al, b, e);
+  const float2 v = fma2(fma2(z, m1, t), m1, s.h), q = fma2(z, m1, p);
+  s.l = add2(s.l, add2(add2(v, q), e));
+  s.h = t;
+}
+__device__ __forceinline__ F2x2 mul2x2(const F2x2& a, const F2x2& b) {
+  F2x2 o;
+  o.h = mul2(a.h, b.h);
+  o.l = fma2(a.h, b.h, mul2(o.h, make_float2(-1.0f, -1.0f)));
+  o.l = fma2(a.h, b.l, o.l);
+  o.l = fma2(a.l, b.h, o.l);
+  return o;
+}
+// The power law's rates (crystal axes) at an FP32 x to about 1e-13, in pairs of
+// FP32 numbers: the first of the last steps only has to reach 1e-11, and FP64
+// rates are 204 of the 990 instructions that bound a solve.  Whole and half
+// exponents, one CRSS per system.  One pair of systems at a time: 128^3 3.5 ms
+// per launch, 3.6 / 3.7 with two / all pairs unrolled (spills), 4.0 with FP64
+// rates; 48^3 0.19 and 0.22 ms, 32^3 67 and 74 us.
+// The result is the FP64 step's after it: against a solve in FP64 throughout the
+// stress is off by 6 to 9e-16 (16^3), 1.0 to 1.7e-15 (32^3), 5.5e-16 (128^3),
+// with FP64 rates here 6 to 9e-16, 1.0 to 1.8e-15, 5.3e-16.
+__device__ __forceinline__ void rates_2xf32(const SlipF& pf, double* dcol, double gamd0, const float (&x)[5],
+                                            double (&ed)[5]) {
+  const float2 zero = dup2(0.0f), m1 = make_float2(-1.0f, -1.0f);
+  F2x2 a[5];
+#pragma unroll
+  for (int i = 0; i < 5; i++) a[i] = F2x2{zero, zero};
+#pragma unroll 1
+  for (int s = 0; s < NSYS / 2; s++) {
+    F2x2 r{zero, zero}, b, p, it;
+#pragma unroll
+    for (int i = 0; i < 5; i++) acc2(r, pf.m[s][i], pf.ml[s][i], dup2(x[i]), zero);
+    const double t0 = ld_at(dcol, LD_TAU + 2 * s), t1 = ld_at(dcol, LD_TAU + 2 * s + 1);
+    it.h = make_float2(f64_to_f32(t0), f64_to_f32(t1));
+    it.l = make_float2(f64_to_f32(t0 - f32_to_f64(it.h.x)), f64_to_f32(t1 - f32_to_f64(it.h.y)));
+    const float2 n = add2(r.h, r.l);
+    r.l = fma2(fma2(r.h, m1, n), m1, r.l);   // l - (n - h)
+    r.h = n;
+    b = r = mul2x2(r, it);
+    int e = pf.nm1;
+    while (!(e & 1)) {
+      b = mul2x2(b, b);
+      e >>= 1;
+    }
+    p = b;
+    while (e >>= 1) {
+      b = mul2x2(b, b);
+      if (e & 1) p = mul2x2(p, b);
+    }
+    if (pf.half) {   // times sqrt |r|
+      b.h = make_float2(sqrtf(fabsf(r.h.x)), sqrtf(fabsf(r.h.y)));
+      auto low = [](float h, float l, float q) {
+        return h != 0.0f ? (fmaf(-q, q, fabsf(h)) + copysignf(1.0f, h) * l) / (2.0f * q) : 0.0f;
+      };
+      b.l = make_float2(low(r.h.x, r.l.x, b.h.x), low(r.h.y, r.l.y, b.h.y));
+      p = mul2x2(p, b);
+    }
+    // |r|^(n-1) r
+    p.l = make_float2(p.h.x < 0.0f ? -p.l.x : p.l.x, p.h.y < 0.0f ? -p.l.y : p.l.y);
+    p.h = make_float2(fabsf(p.h.x), fabsf(p.h.y));
+    r = mul2x2(p, r);
+#pragma unroll
+    for (int i = 0; i < 5; i++) acc2(a[i], pf.m[s][i], pf.ml[s][i], r.h, r.l);
+  }
+#pragma unroll
+  for (int i = 0; i < 5; i++)
+    ed[i] = gamd0 * ((f32_to_f64(a[i].h.x) + f32_to_f64(a[i].h.y)) + (f32_to_f64(a[i].l.x) + f32_to_f64(a[i].l.y)));
 }
 
 // One voxel in FP64.  io: load(lam, eps, ep, R), slip(row), stot(v, out)
@@ -210,6 +291,11 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
       if (nc.flow_off) {
 #pragma unroll
         for (int i = 0; i < 5; i++) ed[i] = 0.0;
+      } else if (LAW == 0 && !GEN && k == 0) {
+        float xs[5];
+#pragma unroll
+        for (int i = 0; i < 5; i++) xs[i] = f64_to_f32(x[i]);   // exact: x is the FP32 start
+        rates_2xf32(pf, dcol, ph.gamd0, xs, ed);
       } else {
         rates_f64<LAW, GEN, IO>(ph, pf, io, dcol, x, ed);
       }

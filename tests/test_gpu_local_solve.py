@@ -102,3 +102,21 @@ def test_steep_first_step_recovers(precision):
     with Solver(capi.params_from_config(cfg, precision=precision), g, p, e) as s:
         r = [s.step() for _ in range(2)]
         assert np.all(np.isfinite(s.field("sig"))) and r[1]["newton_failed"] == 0
+
+
+@pytest.mark.parametrize("nrs", [2.0, 5.5, 10.0, 20.0, 40.5])
+def test_fp64_mode_is_the_all_fp64_iteration(nrs):
+    """The first of the FP64 mode's last steps takes its rates in pairs of FP32 numbers (whole
+    and half exponents); the converged fields are those of the iteration in FP64 throughout
+    (newton_itmax below 50).  Both end with an error far below the tolerance's 1e-10."""
+    cfg = synth.Config(cell_dim=(16, 12, 8), n_grains=6, n_steps=2, seed=19, iter_max=8,
+                       material=synth.Material(nrs=nrs))
+    g, p, e = synth.microstructure(cfg)
+    out = []
+    for kw in ({}, {"newton_itmax": 49}):
+        with Solver(capi.params_from_config(cfg, precision=capi.MTH_FP64, **kw), g, p, e) as s:
+            for _ in range(cfg.n_steps):
+                s.step()
+            out.append((s.field("sig"), s.field("edot"), s.field("crss")))
+    for a, b, tol in zip(*out, (1e-12, 1e-11, 1e-12)):   # edot: amplified by n
+        assert rel_l2(a, b) < tol
