@@ -469,7 +469,7 @@ fft_xg_tma_kernel(const GreenConst gc, const __grid_constant__ CUtensorMap mspec
       T* Ap = reinterpret_cast<T*>(Aq) + i;
 #pragma unroll
       for (int c = 0; c < 6; c++) s[0][c] = Dp[2 * c * SLAB];
-      green_point<T, 1>(gc, kx, y, k0 + kk, L, n1, n2, s, a);
+      green_point<T, 1, true>(gc, kx, y, k0 + kk, L, n1, n2, s, a, i & 1);
 #pragma unroll
       for (int c = 0; c < 6; c++) Dp[2 * c * SLAB] = s[0][c];
 #pragma unroll

@@ -57,6 +57,42 @@ struct GreenDir {
     K[5] = A[4] * A[3] - A[2] * A[5];
     w = -wgt / (A[0] * K[0] + A[5] * K[5] + A[4] * K[4]);
   }
+  // the same by two neighbouring lanes (part 0 and 1 of one wave vector), each
+  // forming half of A and of its cofactors: 24 of the 134 FP64 operations a part
+  // takes.  x + Gamma0 pass at 128^3 0.98 ms, 1.10 with both lanes forming all of
+  // them; 48^3 81 and 89 us, 32^3 29 and 33 us, 16^3 17.5 and 19.1 us.
+  __device__ __forceinline__ void set_pair(const GreenConst& gc, const T (&dir)[3], T wgt, int part) {
+    const unsigned mask = 3u << (threadIdx.x & 30);
+    auto join = [&](const T (&own)[3], T (&all)[6]) {
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        const T o = __shfl_xor_sync(mask, own[j], 1);
+        all[j] = part ? o : own[j];
+        all[3 + j] = part ? own[j] : o;
+      }
+    };
+    T q[6], A[6], t[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) f[i] = dir[i];
+    q[0] = f[0] * f[0];
+    q[1] = f[1] * f[1];
+    q[2] = f[2] * f[2];
+    q[3] = f[1] * f[2];
+    q[4] = f[0] * f[2];
+    q[5] = f[0] * f[1];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      t[j] = GreenTab<T>::a(gc, 3 * part + j, 0) * q[0];
+#pragma unroll
+      for (int k = 1; k < 6; k++) t[j] += GreenTab<T>::a(gc, 3 * part + j, k) * q[k];
+    }
+    join(t, A);
+    t[0] = (part ? A[4] : A[1]) * (part ? A[5] : A[2]) - (part ? A[0] : A[3]) * A[3];
+    t[1] = (part ? A[5] : A[0]) * (part ? A[3] : A[2]) - (part ? A[1] : A[4]) * A[4];
+    t[2] = (part ? A[4] : A[0]) * (part ? A[3] : A[1]) - (part ? A[2] : A[5]) * A[5];
+    join(t, K);
+    w = -wgt / (A[0] * K[0] + A[5] * K[5] + A[4] * K[4]);
+  }
   // real or imaginary parts: s LT components of sigma-hat; adds the LT
   // components of sym(Delta) to d and (21, 02, 10) of its antisymmetric part to a
   __device__ __forceinline__ void apply(const T (&s)[6], T (&d)[6], T (&a)[3]) const {
@@ -94,12 +130,14 @@ struct GreenDir {
 // (src/evolution.c:1402), which equals the transform of the Hermitian part of
 // Delta-hat.  Frequencies as src/init.c:778-786 (the Nyquist index maps to
 // -1/2).  Per launch of the x + Gamma0 pass, before (normalised wave vector,
-// 81 coefficients, one thread per vector) and now: FP64 16^3 44 and 19 us,
-// 32^3 47 and 33 us, 128^3 1.29 and 1.10 ms (FP64 operations bound it);
-// FP32 128^3 51 and 47 us.
-template <typename T, int NP>
+// 81 coefficients, one thread per vector) and now: FP64 16^3 44 and 17.5 us,
+// 32^3 47 and 29 us, 128^3 1.29 and 0.98 ms (FP64 operations bound it);
+// FP32 128^3 51 and 43 us.
+// PAIR: the two parts are on neighbouring lanes of a warp, part says which one
+// this is, and both lanes call.
+template <typename T, int NP, bool PAIR = false>
 __device__ __forceinline__ void green_point(const GreenConst& gc, int kx, int ky, int kz, int n0, int n1, int n2,
-                                            T (&sig)[NP][6], T (&anti)[NP][3]) {
+                                            T (&sig)[NP][6], T (&anti)[NP][3], int part = 0) {
   T dsym[NP][6];
 #pragma unroll
   for (int p = 0; p < NP; p++) {
@@ -133,7 +171,8 @@ __device__ __forceinline__ void green_point(const GreenConst& gc, int kx, int ky
         f[1] = q1 ? f[1] : -f[1];
         f[2] = q2 ? f[2] : -f[2];
       }
-      g.set(gc, f, dirs == 2 ? (T)0.5 : (T)1);
+      if constexpr (PAIR) g.set_pair(gc, f, dirs == 2 ? (T)0.5 : (T)1, part);
+      else g.set(gc, f, dirs == 2 ? (T)0.5 : (T)1);
 #pragma unroll
       for (int p = 0; p < NP; p++) g.apply(sig[p], dsym[p], anti[p]);
     }
