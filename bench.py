@@ -123,38 +123,6 @@ def measured_peaks():
     return 6800.0, "fallback"
 
 
-def fp64_peak_tflops(dev):
-    """FP64 throughput of this GPU, measured here: cuBLAS DGEMM
-    (torch.matmul in float64, 4096^3, best of 5 after 2 warm-up calls, CUDA
-    events on the current stream), in TFLOP/s."""
-    import torch
-    n = 4096
-    g = torch.Generator(device=dev).manual_seed(0)
-    a = torch.randn(n, n, dtype=torch.float64, device=dev, generator=g)
-    b = torch.randn(n, n, dtype=torch.float64, device=dev, generator=g)
-    for _ in range(2):
-        torch.matmul(a, b)
-    best = None
-    for _ in range(5):
-        e0 = torch.cuda.Event(enable_timing=True)
-        e1 = torch.cuda.Event(enable_timing=True)
-        e0.record()
-        torch.matmul(a, b)
-        e1.record()
-        e1.synchronize()
-        t = e0.elapsed_time(e1)
-        best = t if best is None else min(best, t)
-    del a, b
-    return 2.0 * n ** 3 / (best / 1e3) / 1e12
-
-
-# FP64 flops of the mixed mode's Jacobian solve per local Newton step, counted
-# algorithmically (a fused multiply-add is two flops, a reciprocal one): the
-# LDL^T factorisation of the 5x5 Hessian (20 + 20 from the two update sums, 10
-# scalings, 5 pivot reciprocals) and the two triangular solves (20 + 25)
-SOLVE_FP64_FLOPS = 100
-
-
 def traffic_per_launch(kernel):
     """DRAM bytes per launch of a kernel from the committed ncu summary,
     scaled to the 128^3 workload (profiles/traffic.json), or None."""
@@ -271,8 +239,8 @@ def run_gpu(args):
     fb = nv * 55 * (8 if prec == capi.MTH_FP64 else 4) / 1e9   # field planes + half spectra
     out = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
            "ms_per_step": ms_max / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-           "dtype": {capi.MTH_MIXED: "f32 fields + f64 Newton solve", capi.MTH_FP64: "f64",
-                     capi.MTH_MIXED_FAST: "f32", capi.MTH_MIXED_ROOT64: "f32 fields + f64 Newton solve near the root"}[prec],
+           "dtype": {capi.MTH_MIXED: "f32 fields, Newton systems solved to f64 accuracy", capi.MTH_FP64: "f64",
+                     capi.MTH_MIXED_FAST: "f32", capi.MTH_MIXED_ROOT64: "f32 fields, Newton systems solved to f64 accuracy near the root"}[prec],
            "data": describe(cfg)[0],
            "config": {"workload": describe(cfg)[1],
                       "grid": list(cfg.cell_dim), "voxels": nv, "green_iterations": iters,
@@ -291,19 +259,8 @@ def run_gpu(args):
     out["roofline"] = {"bound": "hbm", "kernel": dname, "achieved": achieved, "peak": peak, "unit": "GB/s",
                        "frac": achieved / peak, "peak_source": peak_kind, "traffic": tr,
                        "algorithmic_bytes_per_launch": per_launch_bytes, "ms_per_launch": per_launch_s * 1e3,
-                       "note": "the local Newton is ALU-bound (FP64 solve, FP32 flow rule); its HBM fraction is low "
-                               "by construction"}
-    if prec == capi.MTH_MIXED and dname == "newton":
-        # the local Newton is bound by GB300's FP64 pipe: its FP64 solve flops
-        # against the FP64 throughput measured in this run
-        p64 = fp64_peak_tflops("cuda:%d" % dev_index)
-        steps = float(sum(r["newton_iters"] for r in reps_prof))
-        a64 = SOLVE_FP64_FLOPS * steps / (d["ms"] / 1e3) / 1e12
-        out["roofline"]["fp64"] = {"achieved": a64, "peak": p64, "unit": "TFLOP/s", "frac": a64 / p64,
-                                   "peak_source": "cuBLAS DGEMM 4096^3 measured in this run",
-                                   "flops_per_newton_step": SOLVE_FP64_FLOPS, "newton_steps": steps,
-                                   "note": "algorithmic FP64 flops of the Jacobian solves; the kernel also "
-                                           "runs the FP32 flow rule, residual and Hessian assembly"}
+                       "note": "the local Newton is bound by issue slots (FP64 mode: by the FP64 pipe); its HBM "
+                               "fraction is low by construction"}
     tot_ms = sum(v["ms"] for v in prof.values())
     out["kernels"] = {k: {"ms": round(v["ms"], 3), "share": round(v["ms"] / tot_ms, 4) if tot_ms else None,
                           "launches": v["launches"],
@@ -328,20 +285,20 @@ def run_gpu(args):
         out["fp64"] = {"value": v64, "ms_per_step": ms64 / args.steps, "green_iterations": it64}
         out["mixed_over_fp64"] = value / v64
         out["rel_stress_err_vs_fp64"] = err
-        # opt-in variant with the 5x5 Jacobian solve in FP32 as well
+        # opt-in variant with unrefined FP32 solves of the 5x5 systems
         msf, itf, repsf, _, _, _ = timed_run(capi.MTH_MIXED_FAST, args.steps, args.warmup)
         msf = reduce_max(msf)
         vf = reduce_sum(float(nv) * itf) / (msf / 1e3)
         ef = float(np.abs(repsf[-1]["sig_avg"] - b).max() / np.abs(b).max())
         out["mixed_fast"] = {"value": vf, "ms_per_step": msf / args.steps, "rel_stress_err_vs_fp64": ef,
-                             "note": "MTH_MIXED_FAST: Jacobian solve in FP32 too"}
-        # opt-in variant with the FP64 solve only near the root
+                             "note": "MTH_MIXED_FAST: Jacobian solve in plain FP32"}
+        # opt-in variant that refines the solves only near the root
         msr, itr, repsr, _, _, _ = timed_run(capi.MTH_MIXED_ROOT64, args.steps, args.warmup)
         msr = reduce_max(msr)
         vr = reduce_sum(float(nv) * itr) / (msr / 1e3)
         er = float(np.abs(repsr[-1]["sig_avg"] - b).max() / np.abs(b).max())
         out["mixed_root64"] = {"value": vr, "ms_per_step": msr / args.steps, "rel_stress_err_vs_fp64": er,
-                               "note": "MTH_MIXED_ROOT64: FP64 Jacobian solve only within 1e-3|lambda| of the root"}
+                               "note": "MTH_MIXED_ROOT64: Jacobian solve refined only within 1e-3|lambda| of the root"}
 
     # end to end through the C-ABI with host buffers: create + upload (H2D of
     # the microstructure from pinned memory), K steps each returning the
@@ -470,7 +427,7 @@ def adjoint_measure(dev_index, name="calib64"):
     """Cost of the calibration gradient (mth_adjoint: forward sweep with
     stored states every 10 steps, recomputation, reverse sweep) against a
     plain forward run of the same 64^3 / 256-grain, 50-step tension, mixed
-    precision with the FP64 Jacobian solve.  The target curve comes from the
+    precision.  The target curve comes from the
     forward model at tau0 = 18, thet0 = 280, tau1 = 160, n = 12."""
     import dataclasses
     import torch
@@ -722,8 +679,8 @@ def run_batch(args):
     out = {"metric": "voxel-iterations/s, 64 batched RVEs (24x32^3, 24x48^3, 16x64^3)", "value": value,
            "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
            "ms_per_step": dt * 1e3 / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-           "dtype": {capi.MTH_MIXED: "f32 fields + f64 Newton solve", capi.MTH_FP64: "f64",
-                     capi.MTH_MIXED_FAST: "f32", capi.MTH_MIXED_ROOT64: "f32 fields + f64 Newton solve near the root"}[prec],
+           "dtype": {capi.MTH_MIXED: "f32 fields, Newton systems solved to f64 accuracy", capi.MTH_FP64: "f64",
+                     capi.MTH_MIXED_FAST: "f32", capi.MTH_MIXED_ROOT64: "f32 fields, Newton systems solved to f64 accuracy near the root"}[prec],
            "data": "synthetic: per-RVE seeded periodic Voronoi, grains ~U[32,256], uniform SO(3), "
                    "tau0 ~U[12,20] MPa, n in {8,10,15,20}",
            "config": {"workload": "%d RVEs, uniaxial tension, dt=1e-3" % len(cfgs_all), "rves": len(cfgs_all),

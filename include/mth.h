@@ -39,10 +39,10 @@ typedef enum {
 } mth_status;
 
 typedef enum {
-  MTH_FP64 = 0,       /* all fields, FFTs and the local Newton in FP64 */
+  MTH_FP64 = 0,       /* all fields, FFTs and the local Newton's residual in FP64 */
   MTH_MIXED = 1,      /* FP32 fields/FFT/Green operator/flow rule; Jacobian solves of the local
                          Newton to FP64 accuracy, FP64 error norms and volume averages */
-  MTH_MIXED_FAST = 2, /* as MTH_MIXED but the 5x5 Jacobian solve in FP32 too */
+  MTH_MIXED_FAST = 2, /* as MTH_MIXED but the 5x5 Jacobian solve in plain FP32 */
   MTH_MIXED_ROOT64 = 3 /* as MTH_MIXED but the Jacobian solve to FP64 accuracy only for the Newton
                           steps within 1e-3 |lambda| of the root, in FP32 for the large early steps */
 } mth_precision;
