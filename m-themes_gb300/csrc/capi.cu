@@ -623,6 +623,7 @@ extern "C" mth_status mth_create(const mth_params* p, mth_ctx** out) {
   CKC(cudaMalloc(&c->red, sizeof(double) * 32));
   CKC(cudaMallocHost(&c->red_h, sizeof(double) * 32));
   CKC(cudaMalloc(&c->bk_d, sizeof(IterBook)));
+  CKC(cudaMemset(c->bk_d, 0, sizeof(IterBook)));
   CKC(cudaMallocHost(&c->book_h, sizeof(int) * 4));
   c->book_h[3] = 1;   // source of the live flag's reset
   CKC(cudaMalloc(&c->err_d, sizeof(int)));
@@ -764,7 +765,8 @@ extern "C" mth_status mth_destroy(mth_ctx* c) {
 
 // programmatic dependent launches along the iteration's kernels, outside a
 // batch (whose graph keeps ordinary edges)
-IterIn iter_in(const mth_ctx* c) { return IterIn{c->add_d, c->live_d, c->in_batch ? 0 : c->pdl}; }
+static const int* plain_in(const mth_ctx* c) { return c->plain_step ? &c->bk_d->plain : nullptr; }
+IterIn iter_in(const mth_ctx* c) { return IterIn{c->add_d, c->live_d, c->in_batch ? 0 : c->pdl, plain_in(c)}; }
 
 // gated: the kernel follows the live flag (inside a batch graph)
 mth_status launch_reduce(mth_ctx* c, int width) {
@@ -885,6 +887,7 @@ extern "C" mth_status mth_upload_microstructure(mth_ctx* c, const int* grain, co
     // j != l taken together
     double c4[81];
     m2t4(c->c066, c4);
+    for (int i = 0; i < 81; i++) c->gc.c0f[i] = (float)c4[i];
     const int P[6][2] = {{0, 0}, {1, 1}, {2, 2}, {1, 2}, {0, 2}, {0, 1}};
     auto at = [&](int i, int j, int k, int l) { return c4[((i * 3 + j) * 3 + k) * 3 + l]; };
     for (int p = 0; p < 6; p++)
@@ -967,6 +970,7 @@ extern "C" mth_status mth_upload_microstructure(mth_ctx* c, const int* grain, co
   }
   c->uploaded = 1;
   c->istep = 0;
+  c->plain_next = 1;
   return MTH_OK;
 }
 
@@ -1014,7 +1018,7 @@ static mth_status spin_field(mth_ctx* c) {
   Fields<T>& f = *reinterpret_cast<Fields<T>*>(c->mixed ? (void*)&c->ff : (void*)&c->fd);
   c2<T>* anti = static_cast<c2<T>*>(c->anti);
   auto tw = [&](int a, int d) { return static_cast<const c2<T>*>(c->tw[a][d]); };
-  const IterIn it{nullptr, nullptr};   // no uniform part; always live
+  const IterIn it{nullptr, nullptr, 0, plain_in(c)};   // no uniform part; always live
   const double w = sizeof(T), rp = w * (double)c->nv, kp = 2.0 * w * (double)g.n0 * g.n1 * g.kz;
   const bool tz = !c->tma_off && tma_has(c->tma, 0), ts = !c->tma_off && tma_has(c->tma, 1);
   const T scale = (T)(1.0 / (double)c->nv);
@@ -1235,6 +1239,8 @@ mth_status step_begin(mth_ctx* c) {
   b.err = c->p.err;
   b.e_vm = c->e_vm;
   b.iter_max = c->p.iter_max;
+  c->plain_step = c->plain_next && !c->nc.flow_off && c->mixed && !c->dd;
+  b.plain = c->plain_step;
   b.nan = 0;
   memset(b.ddg, 0, sizeof(b.ddg));
   memset(b.ddg_acum, 0, sizeof(b.ddg_acum));
@@ -1366,6 +1372,7 @@ mth_status step_end(mth_ctx* c, mth_step_report* rep) {
   }
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++) c->disgrad_avg[i][j] = c->disgrad_avg_t[i][j] + c->udot[i][j] * dt;
+  if (!c->nc.flow_off) c->plain_next = c->bk.it_nbad > 0;
   c->istep++;
   return MTH_OK;
 }
@@ -1389,6 +1396,7 @@ extern "C" mth_status mth_step(mth_ctx* c, mth_step_report* rep) {
     while (iter_more(c)) {
       iter_add(c);
       CK(cudaMemcpyAsync(c->add_d, c->add_h, sizeof(double) * 6, cudaMemcpyHostToDevice, c->st));
+      CK(cudaMemcpyAsync(&c->bk_d->plain, &b.plain, sizeof(int), cudaMemcpyHostToDevice, c->st));
       s = c->mixed ? green_iteration<float>(c) : green_iteration<double>(c);
       if (s) return s;
       double red[NPART];

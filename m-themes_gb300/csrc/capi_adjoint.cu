@@ -12,7 +12,7 @@ namespace {
 struct HostCkpt {
   t33 disgrad_avg, disgrad_avg_t, sig_avg, sig_avg1;
   double e_vm, d_vm, s_vm, s_vm1, err_e, err_s, time_tot;
-  int istep;
+  int istep, plain_next;
 };
 constexpr int CKPT_PLANES = 46;   // sig, strain, epsp, edot (6 each), rot 9, crss 12, gamacum 1
 constexpr int SNAP_PLANES = 31;   // before the step: rot 9, crss 12, gamacum 1; after: sig 6, wspin 3
@@ -79,6 +79,7 @@ static mth_status adj_save(mth_ctx* c, AdjRun& run, int slot) {
   memcpy(h.sig_avg1, c->bk.sig_avg1, sizeof(t33));
   h.e_vm = c->e_vm; h.d_vm = c->d_vm; h.s_vm = c->bk.s_vm; h.s_vm1 = c->bk.s_vm1;
   h.err_e = c->bk.err_e; h.err_s = c->bk.err_s; h.time_tot = c->time_tot; h.istep = c->istep;
+  h.plain_next = c->plain_next;
   return MTH_OK;
 }
 
@@ -100,6 +101,7 @@ static mth_status adj_restore(mth_ctx* c, AdjRun& run, int slot) {
   memcpy(c->bk.sig_avg1, h.sig_avg1, sizeof(t33));
   c->e_vm = h.e_vm; c->d_vm = h.d_vm; c->bk.s_vm = h.s_vm; c->bk.s_vm1 = h.s_vm1;
   c->bk.err_e = h.err_e; c->bk.err_s = h.err_s; c->time_tot = h.time_tot; c->istep = h.istep;
+  c->plain_next = h.plain_next;
   return MTH_OK;
 }
 

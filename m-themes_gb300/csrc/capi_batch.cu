@@ -34,6 +34,7 @@ struct mth_batch {
   int* ctl_h = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::vector<NewtonConst> cap_nc;
+  std::vector<int> cap_plain;   // mth_ctx::plain_step of each member
 };
 
 namespace {
@@ -214,7 +215,11 @@ mth_status batch_capture(mth_batch* b) {
   cudaGraphDestroy(g);
   if (s) return s;
   b->cap_nc.resize(n);
-  for (int i = 0; i < n; i++) b->cap_nc[i] = b->rve[i]->nc;
+  b->cap_plain.resize(n);
+  for (int i = 0; i < n; i++) {
+    b->cap_nc[i] = b->rve[i]->nc;
+    b->cap_plain[i] = b->rve[i]->plain_step;
+  }
   return MTH_OK;
 }
 }  // namespace
@@ -321,7 +326,8 @@ extern "C" mth_status mth_batch_step(mth_batch* b, mth_step_report* reports) {
   }
   bool recapture = !b->exec;
   for (int i = 0; i < n && !recapture; i++)
-    recapture = memcmp(&b->cap_nc[i], &b->rve[i]->nc, sizeof(NewtonConst)) != 0;
+    recapture = memcmp(&b->cap_nc[i], &b->rve[i]->nc, sizeof(NewtonConst)) != 0 ||
+                b->cap_plain[i] != b->rve[i]->plain_step;
   if (recapture) {
     mth_status s = batch_capture(b);
     if (s) return s;

@@ -116,6 +116,8 @@ struct mth_ctx {
   bool host_book;     // bookkeeping on the host after every iteration instead (test hook)
   int pdl;            // programmatic dependent launches along the iteration's kernels
   int istep;
+  int plain_next;     // the next step's first iteration runs in plain order (IterBook::plain)
+  int plain_step;     // the step in progress may hold such iterations
   int uploaded;
   // dynamic recrystallisation
   int drx;

@@ -50,6 +50,37 @@ __host__ __device__ constexpr int tl_radix(int n, int idx, int rmax) {
   return 1;
 }
 
+// The plan of a step in plain order (IterIn::plain): the largest radix up to
+// rmax first (16, 8, 4, then 2, then 3).
+__host__ __device__ constexpr int lf_nst(int n, int rmax) {
+  int s = 0;
+  for (int r = rmax; r >= 4; r /= 2)
+    while (n % r == 0) { n /= r; s++; }
+  while (n % 2 == 0) { n /= 2; s++; }
+  while (n % 3 == 0) { n /= 3; s++; }
+  return s;
+}
+__host__ __device__ constexpr int lf_radix(int n, int idx, int rmax) {
+  int s = 0;
+  for (int r = rmax; r >= 4; r /= 2)
+    while (n % r == 0) { if (s == idx) return r; n /= r; s++; }
+  while (n % 2 == 0) { if (s == idx) return 2; n /= 2; s++; }
+  while (n % 3 == 0) { if (s == idx) return 3; n /= 3; s++; }
+  return 1;
+}
+template <bool PLAIN>
+__host__ __device__ constexpr int plan_nst(int n, int rmax) { return PLAIN ? lf_nst(n, rmax) : tl_nst(n, rmax); }
+template <bool PLAIN>
+__host__ __device__ constexpr int plan_radix(int n, int idx, int rmax) {
+  return PLAIN ? lf_radix(n, idx, rmax) : tl_radix(n, idx, rmax);
+}
+__host__ __device__ constexpr bool plans_differ(int n, int rmax, int rmax_plain) {
+  if (tl_nst(n, rmax) != lf_nst(n, rmax_plain)) return true;
+  for (int i = 0; i < tl_nst(n, rmax); i++)
+    if (tl_radix(n, i, rmax) != lf_radix(n, i, rmax_plain)) return true;
+  return false;
+}
+
 // x * W^m for W = exp(sign 2 pi i / 16), m in 0..15, by the values of
 // cos(k pi / 8) (exact constants, no table)
 template <typename T, int M>

@@ -164,12 +164,13 @@ __global__ void __launch_bounds__(256) fft_strided_kernel(c2<T>* __restrict__ sp
 // spectra, Delta = Gamma0 : sigma-hat per k, antisymmetric part added to
 // the spin accumulator, inverse transform along x.  One block: fixed y,
 // kb consecutive kz.
-template <typename T, int NC>
+template <typename T, int NC, bool PLAIN>
 __global__ void __launch_bounds__(256) fft_x_green_kernel(const GreenConst gc, c2<T>* __restrict__ spec, c2<T>* __restrict__ anti_acc,
                                                           long long kplane, int n0_, int n1, int n2, int kzn, int kzs, int kb,
                                                           FftPlan pl, const c2<T>* __restrict__ twf,
                                                           const c2<T>* __restrict__ twi, IterIn it) {
   if (!is_live(it)) return;
+  const bool plain = PLAIN && is_plain(it);
   const int n0 = NC > 0 ? NC : n0_;
   extern __shared__ unsigned char smraw[];
   c2<T>* tw_f = reinterpret_cast<c2<T>*>(smraw);
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(256) fft_x_green_kernel(const GreenConst gc, c
       s[0][c] = v.x;
       s[1][c] = v.y;
     }
-    green_point<T, 2>(gc, kx, y, k0 + kk, n0, n1, n2, s, a);
+    green_point_of<T, PLAIN>(gc, kx, y, k0 + kk, n0, n1, n2, s, a, plain);
 #pragma unroll
     for (int c = 0; c < 6; c++) r[(c * kb + kk) * ls + kx] = mk<T>(s[0][c], s[1][c]);
     const long long o = base + kx * S + kk;
@@ -315,13 +316,23 @@ cudaError_t launch_fft_x_green(const FftGeom& g, const GreenConst& gc, c2<T>* sp
                                const c2<T>* twi, const IterIn& it, cudaStream_t st) {
   const int kb = pick_kb<T>(g.n0, 6, g.smem_budget, 2);
   const size_t sm = s_smem(g.n0, 6 * kb, sizeof(c2<T>), 2);
-  auto k = fft_x_green_kernel<T, 0>;
+  auto k = fft_x_green_kernel<T, 0, false>;
   switch (g.n0) {
-#define MTH_CASE(N) case N: k = fft_x_green_kernel<T, N>; break;
+#define MTH_CASE(N) case N: k = fft_x_green_kernel<T, N, false>; break;
     MTH_CT_SIZES(MTH_CASE)
 #undef MTH_CASE
     default: break;
   }
+  if constexpr (sizeof(T) == 4)
+    if (it.plain) {
+      k = fft_x_green_kernel<T, 0, true>;
+      switch (g.n0) {
+#define MTH_CASE(N) case N: k = fft_x_green_kernel<T, N, true>; break;
+        MTH_CT_SIZES(MTH_CASE)
+#undef MTH_CASE
+        default: break;
+      }
+    }
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   dim3 grid((g.kz + kb - 1) / kb, g.n1);
   k<<<grid, 256, sm, st>>>(gc, spec, anti, g.kplane, g.n0, g.n1, g.n2, g.kz, g.kzs, kb, g.px, twf, twi, it);

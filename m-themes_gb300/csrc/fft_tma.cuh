@@ -166,13 +166,13 @@ __device__ __forceinline__ int tile_slot(int i) {
   if constexpr (SW) return i ^ ((i / B) & (B - 1));
   else return i;
 }
-template <typename T, int N, int QN, int ES, int GS, int NG, int TWM, int SG, int NT, int RMAX, bool SWZ, int S = 0,
-          int NS = 1>
+template <typename T, int N, int QN, int ES, int GS, int NG, int TWM, int SG, int NT, int RMAX, bool SWZ,
+          bool PLAIN = false, int S = 0, int NS = 1>
 __device__ __forceinline__ void tile_fft(c2<T>* d, const c2<T>* __restrict__ tw) {
-  constexpr int NST = tl_nst(N, RMAX);
+  constexpr int NST = plan_nst<PLAIN>(N, RMAX);
   if constexpr (S < NST) {
     constexpr bool SWI = SWZ && S > 0, SWO = SWZ && S + 1 < NST;
-    constexpr int R = tl_radix(N, S, RMAX);
+    constexpr int R = plan_radix<PLAIN>(N, S, RMAX);
     constexpr int NB = N / R;
     constexpr int TWS = N / (NS * R);
     constexpr int TOTAL = NG * NB * QN;
@@ -210,8 +210,27 @@ __device__ __forceinline__ void tile_fft(c2<T>* d, const c2<T>* __restrict__ tw)
       }
     }
     __syncthreads();
-    tile_fft<T, N, QN, ES, GS, NG, TWM, SG, NT, RMAX, SWZ, S + 1, NS * R>(d, tw);
+    tile_fft<T, N, QN, ES, GS, NG, TWM, SG, NT, RMAX, SWZ, PLAIN, S + 1, NS * R>(d, tw);
   }
+}
+
+// FP32 lines that have a second plan, for the iterations in plain order; the
+// kernels with both (PLAIN) run only in steps that may hold such iterations
+template <typename T>
+__host__ __device__ constexpr bool plain_line(int n) {
+  return sizeof(T) == 4 && (n == 16 || n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 256);
+}
+__host__ __device__ constexpr int rmax_plain(int rmax) { return rmax < 16 ? 8 : 16; }
+// tile_fft under the iteration's plan
+template <typename T, int N, int QN, int ES, int GS, int NG, int TWM, int SG, int NT, int RMAX, bool SWZ, bool PLAIN>
+__device__ __forceinline__ void tile_fft_of(c2<T>* d, const c2<T>* __restrict__ tw, bool plain) {
+  if constexpr (PLAIN && plans_differ(N, RMAX, rmax_plain(RMAX))) {
+    if (plain) {
+      tile_fft<T, N, QN, ES, GS, NG, TWM, SG, NT, rmax_plain(RMAX), SWZ, true>(d, tw);
+      return;
+    }
+  }
+  tile_fft<T, N, QN, ES, GS, NG, TWM, SG, NT, RMAX, SWZ>(d, tw);
 }
 
 constexpr int RMAX_Z = 9;     // largest radix: z passes
@@ -287,7 +306,7 @@ __host__ __device__ constexpr int nt_zr(int n, int lb) {
 }
 __host__ __device__ constexpr int nt_zc(int n, int lb) { return nt_tile(n / 2, lb, RMAX_Z, 192, lb * n / 2, lb * n); }
 // r2c: one block = LB consecutive (x,y) lines of one stress component.
-template <typename T, int N, int LB>
+template <typename T, int N, int LB, bool PLAIN>
 __global__ void __launch_bounds__(nt_zr(N, LB)) fft_zr_tma_kernel(
     const T* __restrict__ real, c2<T>* __restrict__ spec, int lines, const c2<T>* __restrict__ tw, IterIn it, int* err) {
   if (!is_live(it)) return;
@@ -306,7 +325,7 @@ __global__ void __launch_bounds__(nt_zr(N, LB)) fft_zr_tma_kernel(
     bulk_load(A, real + row0 * N, bytes, &bar);
   }
   if (!block_wait_loads(&bar, &ok_s, err)) return;
-  tile_fft<T, M, 1, 1, M, LB, 2, -1, NT, RMAX_Z, true>(A, tw);
+  tile_fft_of<T, M, 1, 1, M, LB, 2, -1, NT, RMAX_Z, true, PLAIN>(A, tw, PLAIN && is_plain(it));
   // split step: X_k = (Z_k + conj Z_{M-k})/2 - i W_N^k (Z_k - conj Z_{M-k})/2
   for (int idx = threadIdx.x; idx < LB * KZS; idx += NT) {
     const int l = idx / KZS, k = idx - l * KZS;
@@ -331,7 +350,7 @@ __global__ void __launch_bounds__(nt_zr(N, LB)) fft_zr_tma_kernel(
 // c2r fused with the strain update (MODE 1: field += Re(.)*scale + add[c];
 // MODE 0: field = Re(.)*scale + add[c]).  The imaginary parts of X_0 and
 // X_{N/2} are dropped, as the real part of the reference's complex inverse.
-template <typename T, int N, int LB, int MODE>
+template <typename T, int N, int LB, int MODE, bool PLAIN>
 __global__ void __launch_bounds__(nt_zc(N, LB)) fft_zc_tma_kernel(
     const c2<T>* __restrict__ spec, T* __restrict__ real, int lines, const c2<T>* __restrict__ tw, T scale, IterIn it,
     int* err) {
@@ -363,7 +382,7 @@ __global__ void __launch_bounds__(nt_zc(N, LB)) fft_zc_tma_kernel(
     A[l * M + k] = mk<T>(e.x - o.y, e.y + o.x);   // e + i o
   }
   __syncthreads();
-  tile_fft<T, M, 1, 1, M, LB, 2, +1, NT, RMAX_Z, true>(A, tw);
+  tile_fft_of<T, M, 1, 1, M, LB, 2, +1, NT, RMAX_Z, true, PLAIN>(A, tw, PLAIN && is_plain(it));
   const T ad = it.add ? (T)it.add[comp] : (T)0;
   for (int idx = threadIdx.x; idx < LB * N; idx += NT) {
     const int l = idx / N, z = idx - l * N;
@@ -382,7 +401,7 @@ __global__ void __launch_bounds__(nt_zc(N, LB)) fft_zc_tma_kernel(
 // ------------------------------------------------------- strided passes
 // One block: KB consecutive kz columns of one component at one outer index,
 // lines of L points along y (axis 1) or x (axis 0).
-template <typename T, int L, int KB, int SG>
+template <typename T, int L, int KB, int SG, bool PLAIN>
 __global__ void __launch_bounds__(nt_tile(L, KB, rmax_tile<T>(L, KB))) fft_s_tma_kernel(
     const __grid_constant__ CUtensorMap m, int axis, const c2<T>* __restrict__ tw, IterIn it, int* err) {
   if (!is_live(it)) return;
@@ -399,7 +418,7 @@ __global__ void __launch_bounds__(nt_tile(L, KB, rmax_tile<T>(L, KB))) fft_s_tma
     tma_load4(D, &m, x0, c1, c2i, comp, &bar);
   }
   if (!block_wait_loads(&bar, &ok_s, err)) return;
-  tile_fft<T, L, KB, KB, 0, 1, 1, SG, NT, RM, false>(D, tw);
+  tile_fft_of<T, L, KB, KB, 0, 1, 1, SG, NT, RM, false, PLAIN>(D, tw, PLAIN && is_plain(it));
   fence_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -433,7 +452,7 @@ __host__ __device__ constexpr int slab_elems(int n) {
   return (n + B - 1) / B * B;
 }
 
-template <typename T, int L, int KB>
+template <typename T, int L, int KB, bool PLAIN>
 __global__ void __launch_bounds__(nt_tile(L, 6 * KB, rmax_tile<T>(L, 6 * KB)), xg_min_blocks<T, L, KB>())
 fft_xg_tma_kernel(const GreenConst gc, const __grid_constant__ CUtensorMap mspec,
                   const __grid_constant__ CUtensorMap manti, int n1, int n2, int kz, const c2<T>* __restrict__ twf,
@@ -457,7 +476,8 @@ fft_xg_tma_kernel(const GreenConst gc, const __grid_constant__ CUtensorMap mspec
     for (int c = 0; c < 3; c++) tma_load4(Aq + c * SLAB, &manti, x0, y, 0, c, &bar);
   }
   if (!block_wait_loads(&bar, &ok_s, err)) return;
-  tile_fft<T, L, KB, KB, SLAB, 6, 1, -1, NT, RM, true>(D, twf);
+  const bool plain = PLAIN && is_plain(it);
+  tile_fft_of<T, L, KB, KB, SLAB, 6, 1, -1, NT, RM, true, PLAIN>(D, twf, plain);
   if constexpr (sizeof(T) == 8) {
     // one thread per wave vector and part: twice the warps for the FP64
     // operations, which each sub-partition issues at one per 64 cycles
@@ -486,7 +506,7 @@ fft_xg_tma_kernel(const GreenConst gc, const __grid_constant__ CUtensorMap mspec
         s[0][c] = v.x;
         s[1][c] = v.y;
       }
-      green_point<T, 2>(gc, kx, y, k0 + kk, L, n1, n2, s, a);
+      green_point_of<T, PLAIN>(gc, kx, y, k0 + kk, L, n1, n2, s, a, plain);
 #pragma unroll
       for (int c = 0; c < 6; c++) D[c * SLAB + idx] = mk<T>(s[0][c], s[1][c]);
 #pragma unroll
@@ -494,7 +514,7 @@ fft_xg_tma_kernel(const GreenConst gc, const __grid_constant__ CUtensorMap mspec
     }
   }
   __syncthreads();
-  tile_fft<T, L, KB, KB, SLAB, 6, 1, +1, NT, RM, true>(D, twi);
+  tile_fft_of<T, L, KB, KB, SLAB, 6, 1, +1, NT, RM, true, PLAIN>(D, twi, plain);
   fence_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -600,62 +620,79 @@ static size_t zc_smem(int n, int lb, size_t cb) {
   return cb * (size_t)(((lb * KZS + 15) & ~15) + ((lb * M + 15) & ~15) + lb * M);
 }
 
-template <typename T, int N>
+template <typename T, int N, bool PLAIN>
 static cudaError_t zr_launch(const TmaMaps* t, int ncomp, long long lines, const c2<T>* tw, const IterIn& it,
                              int* err, cudaStream_t st) {
   constexpr int LB = lb_z<T>(N, ZR_ELEMS);
   constexpr int NT = nt_zr(N, LB);
   const size_t sm = zr_smem(N, LB, sizeof(c2<T>));
-  auto k = fft_zr_tma_kernel<T, N, LB>;
+  auto k = fft_zr_tma_kernel<T, N, LB, PLAIN>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   dim3 grid((unsigned)((lines + LB - 1) / LB), ncomp);
   return launch_chain(k, grid, dim3(NT), sm, st, it.pdl, static_cast<const T*>(t->sig),
                       static_cast<c2<T>*>(t->spec), (int)lines, tw, it, err);
 }
 
-template <typename T, int N>
+template <typename T, int N, bool PLAIN>
 static cudaError_t zc_launch(const c2<T>* spec, T* real, int ncomp, long long lines, const c2<T>* tw, T scale,
                              const IterIn& it, int mode, int* err, cudaStream_t st) {
   constexpr int LB = lb_z<T>(N, ZC_ELEMS), NT = nt_zc(N, LB);
   const size_t sm = zc_smem(N, LB, sizeof(c2<T>));
   dim3 grid((unsigned)((lines + LB - 1) / LB), ncomp);
   if (mode) {
-    auto k = fft_zc_tma_kernel<T, N, LB, 1>;
+    auto k = fft_zc_tma_kernel<T, N, LB, 1, PLAIN>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     return launch_chain(k, grid, dim3(NT), sm, st, it.pdl, spec, real, (int)lines, tw, scale, it, err);
   } else {
-    auto k = fft_zc_tma_kernel<T, N, LB, 0>;
+    auto k = fft_zc_tma_kernel<T, N, LB, 0, PLAIN>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     return launch_chain(k, grid, dim3(NT), sm, st, it.pdl, spec, real, (int)lines, tw, scale, it, err);
   }
 }
 
-template <typename T, int L, int KB>
-static cudaError_t s_launch(const CUtensorMap& m, int axis, int ncomp, int nouter, int kzs, int sign,
+template <typename T, int L, int KB, bool PLAIN>
+static cudaError_t s_launch_of(const CUtensorMap& m, int axis, int ncomp, int nouter, int kzs, int sign,
                             const c2<T>* tw, const IterIn& it, int* err, cudaStream_t st) {
   constexpr int NT = nt_tile(L, KB, rmax_tile<T>(L, KB));
   const size_t sm = (size_t)L * KB * sizeof(c2<T>);
   dim3 grid((kzs + KB - 1) / KB, nouter, ncomp);
   if (sign < 0) {
-    auto k = fft_s_tma_kernel<T, L, KB, -1>;
+    auto k = fft_s_tma_kernel<T, L, KB, -1, PLAIN>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     return launch_chain(k, grid, dim3(NT), sm, st, it.pdl, m, axis, tw, it, err);
   }
-  auto k = fft_s_tma_kernel<T, L, KB, +1>;
+  auto k = fft_s_tma_kernel<T, L, KB, +1, PLAIN>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   return launch_chain(k, grid, dim3(NT), sm, st, it.pdl, m, axis, tw, it, err);
 }
 
 template <typename T, int L, int KB>
-static cudaError_t g_launch(const TmaMaps* t, const FftGeom& g, const GreenConst& gc, const c2<T>* twf,
+static cudaError_t s_launch(const CUtensorMap& m, int axis, int ncomp, int nouter, int kzs, int sign,
+                            const c2<T>* tw, const IterIn& it, int* err, cudaStream_t st) {
+  constexpr int RM = rmax_tile<T>(L, KB);
+  if constexpr (plain_line<T>(L) && plans_differ(L, RM, rmax_plain(RM)))
+    if (it.plain) return s_launch_of<T, L, KB, true>(m, axis, ncomp, nouter, kzs, sign, tw, it, err, st);
+  return s_launch_of<T, L, KB, false>(m, axis, ncomp, nouter, kzs, sign, tw, it, err, st);
+}
+
+template <typename T, int L, int KB, bool PLAIN>
+static cudaError_t g_launch_of(const TmaMaps* t, const FftGeom& g, const GreenConst& gc, const c2<T>* twf,
                             const c2<T>* twi, const IterIn& it, int* err, cudaStream_t st) {
   constexpr int NT = nt_tile(L, 6 * KB, rmax_tile<T>(L, 6 * KB));
   const size_t sm = (size_t)9 * slab_elems<T>(L * KB) * sizeof(c2<T>);
-  auto k = fft_xg_tma_kernel<T, L, KB>;
+  auto k = fft_xg_tma_kernel<T, L, KB, PLAIN>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   dim3 grid((g.kzs + KB - 1) / KB, g.n1);
   return launch_chain(k, grid, dim3(NT), sm, st, it.pdl, gc, t->spec_g, t->anti_g, g.n1, g.n2, g.kz, twf, twi, it,
                       err);
+}
+
+template <typename T, int L, int KB>
+static cudaError_t g_launch(const TmaMaps* t, const FftGeom& g, const GreenConst& gc, const c2<T>* twf,
+                            const c2<T>* twi, const IterIn& it, int* err, cudaStream_t st) {
+  if constexpr (plain_line<T>(L))
+    if (it.plain) return g_launch_of<T, L, KB, true>(t, g, gc, twf, twi, it, err, st);
+  return g_launch_of<T, L, KB, false>(t, g, gc, twf, twi, it, err, st);
 }
 
 // the compiled tile widths: FP32 strided 8/16/32, Green 2/4/8; FP64 strided
@@ -684,7 +721,11 @@ cudaError_t tma_fft_z_r2c(const TmaMaps* t, const FftGeom& g, const c2<T>* tw, c
                           cudaStream_t st) {
   const long long lines = (long long)g.n0 * g.n1;
   switch (g.n2) {
-#define MTH_CASE(N) case N: return zr_launch<T, N>(t, 6, lines, tw, it, err, st);
+#define MTH_CASE(N)                                                                                   \
+  case N:                                                                                             \
+    if constexpr (plain_line<T>(N) && plans_differ(N / 2, RMAX_Z, rmax_plain(RMAX_Z)))                \
+      if (it.plain) return zr_launch<T, N, true>(t, 6, lines, tw, it, err, st);                       \
+    return zr_launch<T, N, false>(t, 6, lines, tw, it, err, st);
     MTH_TMA_SIZES(MTH_CASE)
 #undef MTH_CASE
     default: return cudaErrorInvalidValue;
@@ -701,7 +742,11 @@ cudaError_t tma_fft_z_c2r(const TmaMaps* t, const FftGeom& g, int which, const c
   T* mr = static_cast<T*>(which == 1 ? t->wspin : t->strain);
   const int ncomp = which == 1 ? 3 : 6, mode = which == 0;
   switch (g.n2) {
-#define MTH_CASE(N) case N: return zc_launch<T, N>(ms, mr, ncomp, lines, tw, scale, it, mode, err, st);
+#define MTH_CASE(N)                                                                                   \
+  case N:                                                                                             \
+    if constexpr (plain_line<T>(N) && plans_differ(N / 2, RMAX_Z, rmax_plain(RMAX_Z)))                \
+      if (it.plain) return zc_launch<T, N, true>(ms, mr, ncomp, lines, tw, scale, it, mode, err, st); \
+    return zc_launch<T, N, false>(ms, mr, ncomp, lines, tw, scale, it, mode, err, st);
     MTH_TMA_SIZES(MTH_CASE)
 #undef MTH_CASE
     default: return cudaErrorInvalidValue;

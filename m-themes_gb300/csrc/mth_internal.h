@@ -33,6 +33,9 @@ struct IterIn {
   const double* add;
   const int* live;
   int pdl;   // host side: launch the pass as a programmatic dependent of the kernel before it
+  // FP32 modes: not 0 in the iterations in plain order (book.cuh); null in steps
+  // without any, whose kernels have no branch for it
+  const int* plain;
 };
 // The kernels of the Green iteration's chain start with is_live.  Launched
 // as programmatic dependents (launch_chain) they may begin while the kernel
@@ -44,6 +47,7 @@ __device__ __forceinline__ bool is_live(const IterIn& in) {
   chain_wait();
   return !in.live || *in.live;
 }
+__device__ __forceinline__ bool is_plain(const IterIn& in) { return in.plain && *in.plain; }   // after is_live
 #ifdef __CUDACC__
 // Launch of a chain kernel: with pdl, as a programmatic dependent of the
 // previous kernel in the stream (its launch and prologue overlap that
@@ -76,6 +80,7 @@ struct GreenConst {
                       // (chg_basis of C066, src/init.c:376), columns the same pairs (j, l)
   double s066[36];    // S066 = C066^-1 (used at k=0 when ElastBC=0)
   double rn[3];       // 1 / line lengths
+  float c0f[81];      // C0_ijkl, for the FP32 pass in plain order
   float af[6][6];     // single-precision copies for the FP32 pass
   float s066f[36];
   float rnf[3];

@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(256) end_step_kernel(const NewtonConst nc, Fie
       for (int i = 0; i < 6; i++) s6[i] = (TF)f.sig[i * P + v];
       typename SlipOf<LAW, TF, TSt>::type slip;
       SlipOf<LAW, TF, TSt>::load(ph, f, v, slip);
-      rot_to_q_dev<TF>(R, Q);
+      if constexpr (sizeof(TF) == 4) rot_to_q<TF>(R, Q);
+      else rot_to_q_dev<TF>(R, Q);
 #pragma unroll
       for (int i = 0; i < 5; i++) {
         TF a = 0;
@@ -191,13 +192,22 @@ __global__ void __launch_bounds__(256) end_step_kernel(const NewtonConst nc, Fie
             }
           }
           // the hardening matrix is hself on the diagonal, hlat off it (fill_phase):
-          // 24 operations instead of the 12 x 12 products
+          // 24 operations instead of the 12 x 12 products, which FP32 (bound by
+          // memory here) keeps, as it keeps rot_to_q: its roundings decide later
+          // steps of a volume with failed solves (book.cuh)
           const TF hl = ph.nsys > 1 ? cpick<TF>(ph.hard[0][1], ph.hardf[0][1]) : (TF)0;
           const TF hs = cpick<TF>(ph.hard[0][0], ph.hardf[0][0]) - hl, vd = voce / deltgam;
 #pragma unroll
           for (int s = 0; s < NSYS; s++) {
             if (s >= ph.nsys) break;
-            f.crss[s * P + v] = (TSt)((TF)f.crss[s * P + v] + (hl * deltgam + hs * (fabs(gam[s]) * dt)) * vd);
+            if constexpr (sizeof(TF) == 4) {
+              TF dtau = 0;
+#pragma unroll
+              for (int j = 0; j < NSYS; j++) dtau += cpick<TF>(ph.hard[s][j], ph.hardf[s][j]) * fabs(gam[j]) * dt;
+              f.crss[s * P + v] = (TSt)((TF)f.crss[s * P + v] + dtau * voce / deltgam);
+            } else {
+              f.crss[s * P + v] = (TSt)((TF)f.crss[s * P + v] + (hl * deltgam + hs * (fabs(gam[s]) * dt)) * vd);
+            }
           }
           f.gamacum[v] = (TSt)(gamtot + deltgam);
         }

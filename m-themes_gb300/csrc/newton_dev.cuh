@@ -253,10 +253,8 @@ __device__ __forceinline__ bool pivot_positive(T d) {
 
 // LDL^T solve of the packed symmetric positive definite 5x5 matrix A:
 // x = A^-1 b.  Returns false when a pivot is not positive.  NR: pivot
-// reciprocals by pivot_rcp_nr (FP64 solves of the mixed modes).  FLOOR: a
-// pivot below 2^-23 of its diagonal entry, the rounding noise of an
-// FP32-assembled matrix, is raised to that (local_solve.cuh).
-template <typename T, bool NR = false, bool QUAD = false, bool FLOOR = false>
+// reciprocals by pivot_rcp_nr (FP64 solves of the mixed modes).
+template <typename T, bool NR = false, bool QUAD = false>
 __device__ __forceinline__ bool ldl_solve5(const T* A, const T* b, T* x) {
   // U[i][k] = L[i][k] d[k], the column before its scaling by 1/d[k], kept so
   // the updates need no products L d
@@ -267,10 +265,6 @@ __device__ __forceinline__ bool ldl_solve5(const T* A, const T* b, T* x) {
 #pragma unroll
     for (int k = 0; k < 5; k++)
       if (k < j) dj -= U[j][k] * L[j][k];
-    if (FLOOR) {
-      const T low = (T)1.1920928955078125e-7 * A[pk(j, j)];
-      if (!(dj > low)) dj = low;
-    }
     if (!pivot_positive<T, NR>(dj)) return false;
     id[j] = pivot_inv<T, NR, QUAD>(dj);
 #pragma unroll
@@ -318,7 +312,7 @@ __device__ __forceinline__ bool ldl_solve5_wide(const TF* H, const TF* b, TF* x)
     for (int i = 0; i < 15; i++) Hl[i] = f32_to_f64(H[i]);
 #pragma unroll
     for (int i = 0; i < 5; i++) bl[i] = f32_to_f64(b[i]);
-    const bool ok = ldl_solve5<TL, true, true, true>(Hl, bl, pl);
+    const bool ok = ldl_solve5<TL, true, true>(Hl, bl, pl);
 #pragma unroll
     for (int i = 0; i < 5; i++) x[i] = f64_to_f32(pl[i]);
     return ok;
@@ -347,7 +341,7 @@ struct VoxelOut {
 // when the next Newton direction is needed it returns the system H p = -g),
 // nw_pass_b (the move the direction gives) and nw_finish (back to sample
 // axes, error contributions): the damped Newton iteration with every
-// operation in TF, which the FP64 kernels fall back to (solve_full).
+// operation in TF, which the kernels fall back to (solve_full, solve_steep).
 template <typename TF>
 struct NewtonRegs {
   TF K[15], c[5];

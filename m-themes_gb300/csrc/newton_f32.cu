@@ -1,5 +1,6 @@
 // newton_f32.cu -- the local solve of the FP32 modes (newton.cu describes the
 // problem, local_solve.cuh the iteration).
+#include <type_traits>
 #include "newton_dev.cuh"
 
 namespace mth {
@@ -8,20 +9,56 @@ __device__ __noinline__ bool solve5_f64(const float* H, const float* b, float* x
   return ldl_solve5_wide<float, double>(H, b, x);
 }
 
+// A voxel whose solve is not an ordinary one (local_solve.cuh), solved again
+// from lambda by the damped iteration in its plain order of operations.  In the
+// first Green iterations of a volume with a high exponent and a low CRSS (n = 20,
+// 12 MPa) dt dgamma/dtau is more than 1e7 times the elastic compliance, so the
+// rounding of the FP32 Hessian's entries decides whether its factorisation
+// finds a pivot that is not positive; such a solve ends there, keeps its
+// iterate and is counted as failed.  Which voxels those are is therefore a
+// property of this order of operations, and the volume's later iterations
+// start from their stresses.  In the iterations in plain order (book.cuh) every
+// voxel takes it, 1.75 ms a launch at 128^3; elsewhere the test for it and the
+// call cost the kernel 3 % (31.2 against 30.3 ms for 100 launches).
+struct SteepOut {
+  float s6[6], e6[6];
+  VoxelOut<float> o;
+};
+template <int SOLVE, int LAW>
+__device__ __noinline__ void solve_steep(const NewtonConst& nc, const PhaseConst& ph, const Fields<float>& f,
+                                         long long v, SteepOut& out) {
+  const long long P = f.nv;
+  typename SlipOf<LAW, float, float>::type slip;
+  SlipOf<LAW, float, float>::load(ph, f, v, slip);
+  auto load = [&](float* lam6, float* eps6, float* ep6, float* R, bool again) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+      lam6[i] = ld_sel(f.sig + i * P + v, again);
+      eps6[i] = ld_sel(f.strain + i * P + v, again);
+      ep6[i] = ld_sel(f.epsp + i * P + v, again);
+    }
+#pragma unroll
+    for (int i = 0; i < 9; i++) R[i] = ld_sel(f.rot + i * P + v, again);
+  };
+  const float* et = f.etabf + (size_t)f.eclass[v] * ETAB_W;
+  using TL = std::conditional_t<SOLVE == LS_FAST, float, double>;
+  out.o = solve_voxel<float, TL, SOLVE == LS_NEAR_ROOT>(nc, ph, et, slip, load, out.s6, out.e6);
+}
+
 // FP32 modes: one voxel per thread, everything of the solve in FP32 but the
 // systems the refinement leaves to FP64 (local_solve.cuh).  Each thread's
 // K, c and slip-law constants live in its column of shared memory.
 //
 // What bounds it: issue slots (0.70 of the cycles issue; the FP32 pipe is
 // half busy, DRAM a tenth).  128^3, 100 Green iterations, ms (events around
-// each launch): 32.5, 37.4 with one system to an instruction, 103.5 for the
-// earlier kernels, whose blocks stepped their solves in lock step to share the
-// FP64 solves; the FP32-solve mode at 64^3 4.6, 5.2 and 10.7, the
-// dislocation-density law at 96^3 17.2, 17.9 and 31.5.
+// each launch): 31.2; 103.5 for the earlier kernels, whose blocks stepped their
+// solves in lock step to share the FP64 solves; the FP32-solve mode at 64^3 4.6
+// and 10.7, the dislocation-density law at 96^3 17.8 and 31.5.
 template <int SOLVE, int LAW, bool GEN, int MINB>
 __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_constant__ LocalConst lc,
-                                                                 Fields<float> f, double* __restrict__ partials,
-                                                                 IterIn it) {
+                                                                 const __grid_constant__ NewtonConst nc,
+                                                                 const __grid_constant__ Fields<float> f,
+                                                                 double* __restrict__ partials, IterIn it) {
   if (!is_live(it)) return;
   extern __shared__ __align__(16) float ls_sm[];
   float* col = ls_sm + threadIdx.x;
@@ -88,60 +125,75 @@ __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_co
 #pragma unroll
         for (int s = 0; s < 3 * NSYS; s++) ls_at(col, LS_LAW + s) = f.ddc[s * P + v];
       }
-      const SolveF32 o =
-          solve_f32<SOLVE, LAW, GEN, false>(lc, ph, col, et[ET_STOT_MIN], ref2, h, dh, x, ed);
-      // back to sample axes; the inputs are read again rather than held
-      // through the solve
-      float lam[6], u[6], R[9], ss[5], es[5];
+      SolveF32 o{0, false, true};
+      if (LAW == 1 || !is_plain(it))
+        o = solve_f32<SOLVE, LAW, GEN, false>(lc, ph, col, et[ET_STOT_MIN], ref2, h, dh, x, ed);
+      if (o.steep) {
+        SteepOut r;
+        solve_steep<SOLVE, LAW>(nc, nc.ph[GEN ? jph : 0], f, v, r);
 #pragma unroll
-      for (int i = 0; i < 9; i++) R[i] = ld_again(f.rot + i * P + v);
-      {
-        float2 xe[5], se[5];
+        for (int i = 0; i < 6; i++) {
+          f.sig[i * P + v] = r.s6[i];
+          f.edot[i * P + v] = r.e6[i];
+          acc[2 + i] = r.s6[i];
+        }
+        acc[0] = r.o.conv_s;
+        acc[1] = r.o.conv_e;
+        acc[14] = (float)r.o.iters;
+        acc[15] = (float)r.o.failed;
+      } else {
+        // back to sample axes; the inputs are read again rather than held
+        // through the solve
+        float lam[6], u[6], R[9], ss[5], es[5];
 #pragma unroll
-        for (int i = 0; i < 5; i++) xe[i] = make_float2(x[i], ed[i]);
-        dev_to_sample2(R, xe, se);
+        for (int i = 0; i < 9; i++) R[i] = ld_again(f.rot + i * P + v);
+        {
+          float2 xe[5], se[5];
+#pragma unroll
+          for (int i = 0; i < 5; i++) xe[i] = make_float2(x[i], ed[i]);
+          dev_to_sample2(R, xe, se);
+#pragma unroll
+          for (int i = 0; i < 5; i++) {
+            ss[i] = se[i].x;
+            es[i] = se[i].y;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+          lam[i] = ld_again(f.sig + i * P + v);
+          u[i] = ld_again(f.epsp + i * P + v) - ld_again(f.strain + i * P + v);
+        }
+        float cs = dh * dh, ce;
+        {
+          const float de = fmaf(et[ET_SEL_HH], h, u[5]);
+          ce = de * de;
+        }
 #pragma unroll
         for (int i = 0; i < 5; i++) {
-          ss[i] = se[i].x;
-          es[i] = se[i].y;
+          const float ds = ss[i] - lam[i];
+          cs = fmaf(ds, ds, cs);
+          float de = fmaf(lc.dt, es[i], u[i]);
+#pragma unroll
+          for (int j = 0; j < 5; j++) de = fmaf(et[ET_SEL + pk5s(i, j)], ss[j], de);
+          ce = fmaf(de, de, ce);
         }
-      }
 #pragma unroll
-      for (int i = 0; i < 6; i++) {
-        lam[i] = ld_again(f.sig + i * P + v);
-        u[i] = ld_again(f.epsp + i * P + v) - ld_again(f.strain + i * P + v);
+        for (int i = 0; i < 5; i++) {
+          f.sig[i * P + v] = ss[i];
+          f.edot[i * P + v] = es[i];
+          acc[2 + i] = ss[i];
+        }
+        f.sig[5 * P + v] = h;
+        f.edot[5 * P + v] = 0.0f;
+        acc[7] = h;
+        acc[0] = sqrtf(cs);
+        acc[1] = sqrtf(ce);
+        acc[14] = (float)o.it;   // small integers: exact
       }
-      float cs = dh * dh, ce;
-      {
-        const float de = fmaf(et[ET_SEL_HH], h, u[5]);
-        ce = de * de;
-      }
-#pragma unroll
-      for (int i = 0; i < 5; i++) {
-        const float ds = ss[i] - lam[i];
-        cs = fmaf(ds, ds, cs);
-        float de = fmaf(lc.dt, es[i], u[i]);
-#pragma unroll
-        for (int j = 0; j < 5; j++) de = fmaf(et[ET_SEL + pk5s(i, j)], ss[j], de);
-        ce = fmaf(de, de, ce);
-      }
-#pragma unroll
-      for (int i = 0; i < 5; i++) {
-        f.sig[i * P + v] = ss[i];
-        f.edot[i * P + v] = es[i];
-        acc[2 + i] = ss[i];
-      }
-      f.sig[5 * P + v] = h;
-      f.edot[5 * P + v] = 0.0f;
-      acc[7] = h;
-      acc[0] = sqrtf(cs);
-      acc[1] = sqrtf(ce);
       if (GEN && jph == 0) {
 #pragma unroll
         for (int i = 0; i < 6; i++) acc[8 + i] = acc[2 + i];
       }
-      acc[14] = (float)o.it;   // small integers: exact
-      acc[15] = o.failed ? 1.0f : 0.0f;
     } else {
 #pragma unroll
       for (int i = 0; i < 6; i++) {
@@ -164,28 +216,30 @@ __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_co
 #endif
 
 template <int SOLVE, int LAW, bool GEN, int MINB>
-static cudaError_t launch_f32(const LocalConst& lc, const Fields<float>& f, double* partials, const IterIn& it,
-                              cudaStream_t st) {
+static cudaError_t launch_f32(const LocalConst& lc, const NewtonConst& nc, const Fields<float>& f, double* partials,
+                              const IterIn& it, cudaStream_t st) {
   const int nt = newton_threads(f.nv, false);
   return launch_chain(newton_f32_kernel<SOLVE, LAW, GEN, MINB>, dim3(newton_blocks(f.nv, false)), dim3(nt),
-                      sizeof(float) * LS_NT * ls_rows<LAW, GEN>(), st, it.pdl, lc, f, partials, it);
+                      sizeof(float) * LS_NT * ls_rows<LAW, GEN>(), st, it.pdl, lc, nc, f, partials, it);
 }
 template <int SOLVE, int LAW, int MINB>
-static cudaError_t launch_f32_gen(bool plain, const LocalConst& lc, const Fields<float>& f, double* partials,
-                                  const IterIn& it, cudaStream_t st) {
-  return plain ? launch_f32<SOLVE, LAW, false, MINB>(lc, f, partials, it, st)
-               : launch_f32<SOLVE, LAW, true, MINB>(lc, f, partials, it, st);
+static cudaError_t launch_f32_gen(bool plain, const LocalConst& lc, const NewtonConst& nc, const Fields<float>& f,
+                                  double* partials, const IterIn& it, cudaStream_t st) {
+  return plain ? launch_f32<SOLVE, LAW, false, MINB>(lc, nc, f, partials, it, st)
+               : launch_f32<SOLVE, LAW, true, MINB>(lc, nc, f, partials, it, st);
 }
-cudaError_t launch_newton_f32(int mixed, const NewtonConst& nc, const Fields<float>& f, double* partials,
+cudaError_t launch_newton_f32(int mixed, const NewtonConst& nc_in, const Fields<float>& f, double* partials,
                               const IterIn& it, cudaStream_t st, int law) {
   LocalConst lc;
-  fill_local(nc, false, lc);
+  fill_local(nc_in, false, lc);
+  NewtonConst nc = nc_in;
+  fill_float_consts(nc);
   const bool plain = plain_phase(nc, lc);
   // dislocation-density law: refined solves at every step in all mixed modes
-  if (law == 1) return launch_f32_gen<LS_REFINED, 1, MTH_DD_MINB>(nc.ph1_only != 0, lc, f, partials, it, st);
-  if (mixed == 2) return launch_f32_gen<LS_FAST, 0, MTH_F32_MINB>(plain, lc, f, partials, it, st);
-  if (mixed == 3) return launch_f32_gen<LS_NEAR_ROOT, 0, MTH_F32_MINB>(plain, lc, f, partials, it, st);
-  return launch_f32_gen<LS_REFINED, 0, MTH_F32_MINB>(plain, lc, f, partials, it, st);
+  if (law == 1) return launch_f32_gen<LS_REFINED, 1, MTH_DD_MINB>(nc.ph1_only != 0, lc, nc, f, partials, it, st);
+  if (mixed == 2) return launch_f32_gen<LS_FAST, 0, MTH_F32_MINB>(plain, lc, nc, f, partials, it, st);
+  if (mixed == 3) return launch_f32_gen<LS_NEAR_ROOT, 0, MTH_F32_MINB>(plain, lc, nc, f, partials, it, st);
+  return launch_f32_gen<LS_REFINED, 0, MTH_F32_MINB>(plain, lc, nc, f, partials, it, st);
 }
 
 }  // namespace mth
