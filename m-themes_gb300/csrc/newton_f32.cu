@@ -19,7 +19,7 @@ __device__ __noinline__ bool solve5_f64(const float* H, const float* b, float* x
 // property of this order of operations, and the volume's later iterations
 // start from their stresses.  In the iterations in plain order (book.cuh) every
 // voxel takes it, 1.75 ms a launch at 128^3; elsewhere the test for it and the
-// call cost the kernel 3 % (31.2 against 30.3 ms for 100 launches).
+// call cost the kernel 3 % (0.9 ms of 100 launches).
 struct SteepOut {
   float s6[6], e6[6];
   VoxelOut<float> o;
@@ -51,7 +51,7 @@ __device__ __noinline__ void solve_steep(const NewtonConst& nc, const PhaseConst
 //
 // What bounds it: issue slots (0.70 of the cycles issue; the FP32 pipe is
 // half busy, DRAM a tenth).  128^3, 100 Green iterations, ms (events around
-// each launch): 31.2; 103.5 for the earlier kernels, whose blocks stepped their
+// each launch): 34.7; 103.5 for the earlier kernels, whose blocks stepped their
 // solves in lock step to share the FP64 solves; the FP32-solve mode at 64^3 4.6
 // and 10.7, the dislocation-density law at 96^3 17.8 and 31.5.
 template <int SOLVE, int LAW, bool GEN, int MINB>
