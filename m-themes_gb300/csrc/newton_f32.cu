@@ -9,8 +9,9 @@ __device__ __noinline__ bool solve5_f64(const float* H, const float* b, float* x
   return ldl_solve5_wide<float, double>(H, b, x);
 }
 
-// A voxel whose solve is not an ordinary one (local_solve.cuh), solved again
-// from lambda by the damped iteration in its plain order of operations.  In the
+// A voxel whose solve is not an ordinary one (local_solve.cuh), or with a CRSS
+// that softened to zero or below, solved from lambda by the damped iteration in
+// its plain order of operations.  In the
 // first Green iterations of a volume with a high exponent and a low CRSS (n = 20,
 // 12 MPa) dt dgamma/dtau is more than 1e7 times the elastic compliance, so the
 // rounding of the FP32 Hessian's entries decides whether its factorisation
@@ -51,7 +52,7 @@ __device__ __noinline__ void solve_steep(const NewtonConst& nc, const PhaseConst
 //
 // What bounds it: issue slots (0.70 of the cycles issue; the FP32 pipe is
 // half busy, DRAM a tenth).  128^3, 100 Green iterations, ms (events around
-// each launch): 34.7; 103.5 for the earlier kernels, whose blocks stepped their
+// each launch): 35.1; 103.5 for the earlier kernels, whose blocks stepped their
 // solves in lock step to share the FP64 solves; the FP32-solve mode at 64^3 4.6
 // and 10.7, the dislocation-density law at 96^3 17.8 and 31.5.
 template <int SOLVE, int LAW, bool GEN, int MINB>
@@ -112,13 +113,17 @@ __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_co
         store_k(Q, S, col);
       }
       if constexpr (LAW == 0) {
+        const int ns = nc.ph[GEN ? jph : 0].nsys;
 #pragma unroll
         for (int s = 0; s < NSYS; s++) {
           const float t = f.crss[s * P + v];
-          ls_at(col, LS_LAW + s) = t > 0.0f ? rcp_f32(t) : 0.0f;   // 0 in the slots past nsys
+          // 0 in the slots past nsys; a CRSS of an active system that softened to zero
+          // or below gives no direction (steep)
+          const float none = s < ns ? __int_as_float(0x7fffffff) : 0.0f;
+          ls_at(col, LS_LAW + s) = t > 0.0f ? rcp_f32(t) : none;
           if (GEN) {
             const float tb = t + ph.tau_off;
-            ls_at(col, LS_LAW + NSYS + s) = t > 0.0f ? rcp_f32(tb) : 0.0f;
+            ls_at(col, LS_LAW + NSYS + s) = t > 0.0f && tb > 0.0f ? rcp_f32(tb) : none;
           }
         }
       } else {
