@@ -59,7 +59,11 @@ __device__ __noinline__ void solve_full(const NewtonConst& nc, const PhaseConst&
   io.failed = o.failed;
 }
 
-// 1/t, positive t: pivot_rcp_nr and a residual correction
+// what rcp_f64 takes: positive, normal, with a normal reciprocal
+__device__ __forceinline__ bool rcp_ok(double t) {
+  return (unsigned)__double2hiint(t) - 0x00100000u < 0x7fd00000u - 0x00100000u;
+}
+// 1/t: pivot_rcp_nr, which reads no sign, and a residual correction
 __device__ __forceinline__ double rcp_f64(double t) {
   const double x = pivot_rcp_nr<false>(t);
   return fma(x, fma(-t, x, 1.0), x);
@@ -260,13 +264,16 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
 #pragma unroll
       for (int s = 0; s < NSYS; s++) {
         const double t = io.slip(s);
-        const bool on = __double2hiint(t) > 0;
+        const bool on = rcp_ok(t);
         ok = ok && (on || s >= ph.nsys);   // a CRSS that is not positive: every pass in FP64
         const double ti = on ? rcp_f64(t) : 0.0;
         ld_at(dcol, LD_TAU + s) = ti;
         ls_at(col, LS_LAW + s) = f64_to_f32(ti);
         if (GEN) {
-          const double tb = on ? rcp_f64(t + ph.tau_back_minus_fwd) : 0.0;
+          const double tbk = t + ph.tau_back_minus_fwd;
+          const bool onb = on && rcp_ok(tbk);
+          ok = ok && (onb || s >= ph.nsys);   // the backward one too
+          const double tb = onb ? rcp_f64(tbk) : 0.0;
           ld_at(dcol, LD_TAU + NSYS + s) = tb;
           ls_at(col, LS_LAW + NSYS + s) = f64_to_f32(tb);
         }

@@ -29,3 +29,24 @@ def test_softened_system_is_reported(precision):
         s.step()
         with pytest.raises(capi.MthError):
             s.step()
+
+
+@pytest.mark.parametrize("off", [-4.0, -12.0])
+def test_array_points_below_the_backward_offset(off):
+    """Points whose CRSS lies below tau0f - tau0b: the result is the iteration's with every
+    pass in FP64 (a cap below 50 selects it)."""
+    import pyoracle
+    from test_oracle_cpu import random_states
+    cfg = synth.Config(cell_dim=(8, 8, 8), n_grains=4)
+    p = capi.params_from_config(cfg)
+    c066 = pyoracle.Oracle(p, *synth.microstructure(cfg), nthreads=2).c066()
+    p.phase[0].tau0b = p.phase[0].tau0f + off
+    st = [np.array(x) for x in random_states(65, np.random.default_rng(11), cfg)]
+    st[4][::3] *= 0.1
+    assert (st[4] + off < 0).any() and (st[4] + off > 0).any()
+    p.newton_itmax = 49
+    full = local_solve(p, c066, *st)
+    p.newton_itmax = 0
+    got = local_solve(p, c066, *st)
+    for a, b in zip(got[:2], full[:2]):
+        assert np.abs(a - b).max() <= 1e-8 * np.abs(b).max()   # both solve to 1e-10 |lambda|
