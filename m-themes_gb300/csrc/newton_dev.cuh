@@ -695,11 +695,11 @@ __device__ __forceinline__ void block_reduce_smem(const TV (&v)[W], double* out)
 }
 
 // Sums over a warp of NC values per lane, in FP64 in a fixed order: rows[c]
-// of the warp's 32 columns (row stride LS_NT) hold the values; 32/NC lanes
+// of the warp's 32 columns (row stride LD) hold the values; 32/NC lanes
 // per component each add their share, so a warp issues 11 (NC = 10) or 16
 // (NC = 16) FP64 additions.  Lane c < NC returns component c's sum.  The
 // read order is rotated by the component, so the lanes hit distinct banks.
-template <typename TV, int NC>
+template <typename TV, int NC, int LD>
 __device__ __forceinline__ double warp_sums(const TV* rows, int lane) {
   constexpr int NP = 32 / NC, LEN = (32 + NP - 1) / NP;
   const int comp = lane % NC, part = lane / NC;
@@ -710,7 +710,7 @@ __device__ __forceinline__ double warp_sums(const TV* rows, int lane) {
       int j = k + comp;
       j -= j >= LEN ? LEN : 0;
       const int i = part * LEN + j;
-      if (32 % LEN == 0 || i < 32) a += to_f64(rows[comp * LS_NT + i]);
+      if (32 % LEN == 0 || i < 32) a += to_f64(rows[comp * LD + i]);
     }
   }
   double b = a;
@@ -723,16 +723,17 @@ __device__ __forceinline__ double warp_sums(const TV* rows, int lane) {
 // !GEN (phase 1 the only crystal phase): the phase-1 stress sums (8..13)
 // are the total ones (2..7), added once and written twice.  rows: this
 // warp's columns of shared memory, its solve's data no longer needed.
-template <typename TV, bool GEN>
-__device__ __forceinline__ void newton_block_sums(const TV (&v)[NPART], TV* col, double* __restrict__ out) {
+template <typename TV, bool GEN, int LD>
+__device__ __forceinline__ void newton_block_sums(const TV (&v)[NPART], const Column<TV, LD>& col,
+                                                  double* __restrict__ out) {
   constexpr int NC = GEN ? 16 : 10;
-  __shared__ double wsum[LS_NT / 32][NPART];
+  __shared__ double wsum[LD / 32][NPART];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < NC; c++) col[c * LS_NT] = v[!GEN && c >= 8 ? c + 6 : c];
+  for (int c = 0; c < NC; c++) col(c) = v[!GEN && c >= 8 ? c + 6 : c];
   __syncwarp();
-  const double a = warp_sums<TV, NC>(col - lane, lane);
+  const double a = warp_sums<TV, NC, LD>(col.p - lane, lane);
   if (lane < NC) {
     if (GEN || lane < 8) wsum[w][lane] = a;
     else wsum[w][lane + 6] = a;

@@ -5,6 +5,8 @@
 
 namespace mth {
 
+constexpr int F32_NT = 128;   // threads of the largest block
+
 __device__ __noinline__ bool solve5_f64(const float* H, const float* b, float* x) {
   return ldl_solve5_wide<float, double>(H, b, x);
 }
@@ -56,13 +58,13 @@ __device__ __noinline__ void solve_steep(const NewtonConst& nc, const PhaseConst
 // solves in lock step to share the FP64 solves; the FP32-solve mode at 64^3 4.6
 // and 10.7, the dislocation-density law at 96^3 17.8 and 31.5.
 template <int SOLVE, int LAW, bool GEN, int MINB>
-__global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_constant__ LocalConst lc,
+__global__ void __launch_bounds__(F32_NT, MINB) newton_f32_kernel(const __grid_constant__ LocalConst lc,
                                                                  const __grid_constant__ NewtonConst nc,
                                                                  const __grid_constant__ Fields<float> f,
                                                                  double* __restrict__ partials, IterIn it) {
   if (!is_live(it)) return;
   extern __shared__ __align__(16) float ls_sm[];
-  float* col = ls_sm + threadIdx.x;
+  const Column<float, F32_NT> col{ls_sm + threadIdx.x};
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long P = f.nv;
   float acc[NPART];
@@ -105,7 +107,7 @@ __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_co
             b = fmaf(Q[i * 5 + j], u[j], b);
           }
           x[i] = a;
-          ls_at(col, LS_C + i) = b;
+          col(LS_C + i) = b;
         }
         float S[15];
 #pragma unroll
@@ -120,15 +122,15 @@ __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_co
           // 0 in the slots past nsys; a CRSS of an active system that softened to zero
           // or below gives no direction (steep)
           const float none = s < ns ? __int_as_float(0x7fffffff) : 0.0f;
-          ls_at(col, LS_LAW + s) = t > 0.0f ? rcp_f32(t) : none;
+          col(LS_LAW + s) = t > 0.0f ? rcp_f32(t) : none;
           if (GEN) {
             const float tb = t + ph.tau_off;
-            ls_at(col, LS_LAW + NSYS + s) = t > 0.0f && tb > 0.0f ? rcp_f32(tb) : none;
+            col(LS_LAW + NSYS + s) = t > 0.0f && tb > 0.0f ? rcp_f32(tb) : none;
           }
         }
       } else {
 #pragma unroll
-        for (int s = 0; s < 3 * NSYS; s++) ls_at(col, LS_LAW + s) = f.ddc[s * P + v];
+        for (int s = 0; s < 3 * NSYS; s++) col(LS_LAW + s) = f.ddc[s * P + v];
       }
       SolveF32 o{0, false, true};
       if (LAW == 1 || !is_plain(it))
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(LS_NT, MINB) newton_f32_kernel(const __grid_co
       }
     }
   }
-  newton_block_sums<float, GEN>(acc, col, partials);
+  newton_block_sums<float, GEN, F32_NT>(acc, col, partials);
 }
 
 // Blocks of 128 threads per SM the kernels are compiled for.  100 launches,
@@ -225,7 +227,7 @@ static cudaError_t launch_f32(const LocalConst& lc, const NewtonConst& nc, const
                               const IterIn& it, cudaStream_t st) {
   const int nt = newton_threads(f.nv, false);
   return launch_chain(newton_f32_kernel<SOLVE, LAW, GEN, MINB>, dim3(newton_blocks(f.nv, false)), dim3(nt),
-                      sizeof(float) * LS_NT * ls_rows<LAW, GEN>(), st, it.pdl, lc, nc, f, partials, it);
+                      sizeof(float) * F32_NT * ls_rows<LAW, GEN>(), st, it.pdl, lc, nc, f, partials, it);
 }
 template <int SOLVE, int LAW, int MINB>
 static cudaError_t launch_f32_gen(bool plain, const LocalConst& lc, const NewtonConst& nc, const Fields<float>& f,

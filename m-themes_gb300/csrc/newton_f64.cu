@@ -1,10 +1,13 @@
 // newton_f64.cu -- the local solve of the FP64 mode and of the array entry
 // points (newton.cu describes the problem).
 #include <atomic>
-#define LS_COLUMNS 64   // threads of the largest block
 #include "newton_dev.cuh"
 
 namespace mth {
+
+constexpr int F64_NT = 64;   // threads of the largest block
+using FCol = Column<float, F64_NT>;
+using DCol = Column<double, F64_NT>;
 
 // ---- FP64 mode
 // GB300 issues FP64 at 1/64 of the FP32 rate, so what bounds a solve is the
@@ -74,12 +77,11 @@ constexpr int LD_Q = 0, LD_TAU = 25;
 template <int LAW, bool GEN>
 __host__ __device__ constexpr int ld_rows() { return LD_TAU + (LAW == 1 ? 0 : GEN ? 2 * NSYS : NSYS); }
 template <int LAW, bool GEN>
-constexpr size_t f64_smem() { return (size_t)LS_NT * (4 * ls_rows<LAW, GEN>() + 8 * ld_rows<LAW, GEN>()); }
-__device__ __forceinline__ double& ld_at(double* col, int row) { return col[row * LS_NT]; }
+constexpr size_t f64_smem() { return (size_t)F64_NT * (4 * ls_rows<LAW, GEN>() + 8 * ld_rows<LAW, GEN>()); }
 
 // rates (crystal axes) at x in FP64
 template <int LAW, bool GEN, typename IO>
-__device__ __forceinline__ void rates_f64(const PhaseConst& ph, const SlipF& pf, const IO& io, double* dcol,
+__device__ __forceinline__ void rates_f64(const PhaseConst& ph, const SlipF& pf, const IO& io, const DCol& dcol,
                                           const double (&x)[5], double (&ed)[5]) {
 #pragma unroll
   for (int i = 0; i < 5; i++) ed[i] = 0.0;
@@ -89,8 +91,8 @@ __device__ __forceinline__ void rates_f64(const PhaseConst& ph, const SlipF& pf,
     for (int s = 0; s < NSYS; s++) {
       const double* m = ph.m_xt[s];
       const double rss = m[0] * x[0] + m[1] * x[1] + m[2] * x[2] + m[3] * x[3] + m[4] * x[4];
-      double t = ld_at(dcol, LD_TAU + s);
-      if (GEN && __double2hiint(rss) < 0) t = ld_at(dcol, LD_TAU + NSYS + s);
+      double t = dcol(LD_TAU + s);
+      if (GEN && __double2hiint(rss) < 0) t = dcol(LD_TAU + NSYS + s);
       r[s] = rss * t;
       b[s] = fabs(r[s]);
     }
@@ -149,7 +151,7 @@ __device__ __forceinline__ F2x2 mul2x2(const F2x2& a, const F2x2& b) {
 // The result is the FP64 step's after it: against a solve in FP64 throughout the
 // stress is off by 6 to 9e-16 (16^3), 1.0 to 1.7e-15 (32^3), 5.5e-16 (128^3),
 // with FP64 rates here 6 to 9e-16, 1.0 to 1.8e-15, 5.3e-16.
-__device__ __forceinline__ void rates_2xf32(const SlipF& pf, double* dcol, double gamd0, const float (&x)[5],
+__device__ __forceinline__ void rates_2xf32(const SlipF& pf, const DCol& dcol, double gamd0, const float (&x)[5],
                                             double (&ed)[5]) {
   const float2 zero = dup2(0.0f), m1 = make_float2(-1.0f, -1.0f);
   F2x2 a[5];
@@ -160,7 +162,7 @@ __device__ __forceinline__ void rates_2xf32(const SlipF& pf, double* dcol, doubl
     F2x2 r{zero, zero}, b, p, it;
 #pragma unroll
     for (int i = 0; i < 5; i++) acc2(r, pf.m[s][i], pf.ml[s][i], dup2(x[i]), zero);
-    const double t0 = ld_at(dcol, LD_TAU + 2 * s), t1 = ld_at(dcol, LD_TAU + 2 * s + 1);
+    const double t0 = dcol(LD_TAU + 2 * s), t1 = dcol(LD_TAU + 2 * s + 1);
     it.h = make_float2(f64_to_f32(t0), f64_to_f32(t1));
     it.l = make_float2(f64_to_f32(t0 - f32_to_f64(it.h.x)), f64_to_f32(t1 - f32_to_f64(it.h.y)));
     const float2 n = add2(r.h, r.l);
@@ -206,7 +208,7 @@ struct OutF64 {
 };
 template <int LAW, bool GEN, typename IO>
 __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalConst& lc, const PhaseConst& ph,
-                                          const SlipF& pf, IO& io, float* col, double* dcol, OutF64& out) {
+                                          const SlipF& pf, IO& io, const FCol& col, const DCol& dcol, OutF64& out) {
   double x[5], c[5], ed[5], h, dh;
   float ref2;
   bool ok = nc.itmax >= 50;
@@ -223,7 +225,7 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
         rot_to_q_dev<double>(R, Q);
         io.set_q(Q);
 #pragma unroll
-        for (int i = 0; i < 25; i++) ld_at(dcol, LD_Q + i) = Q[i];
+        for (int i = 0; i < 25; i++) dcol(LD_Q + i) = Q[i];
         float Rf[9], Qf[25], S[15];
 #pragma unroll
         for (int i = 0; i < 9; i++) Rf[i] = f64_to_f32(R[i]);
@@ -251,13 +253,13 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
         double a = 0, b = 0;
 #pragma unroll
         for (int j = 0; j < 5; j++) {
-          const double q = ld_at(dcol, LD_Q + i * 5 + j);
+          const double q = dcol(LD_Q + i * 5 + j);
           a += q * lam[j];
           b += q * x[j];
         }
         xf[i] = f64_to_f32(a);
         c[i] = b;
-        ls_at(col, LS_C + i) = f64_to_f32(b);
+        col(LS_C + i) = f64_to_f32(b);
       }
     }
     if constexpr (LAW == 0) {
@@ -267,20 +269,20 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
         const bool on = rcp_ok(t);
         ok = ok && (on || s >= ph.nsys);   // a CRSS that is not positive: every pass in FP64
         const double ti = on ? rcp_f64(t) : 0.0;
-        ld_at(dcol, LD_TAU + s) = ti;
-        ls_at(col, LS_LAW + s) = f64_to_f32(ti);
+        dcol(LD_TAU + s) = ti;
+        col(LS_LAW + s) = f64_to_f32(ti);
         if (GEN) {
           const double tbk = t + ph.tau_back_minus_fwd;
           const bool onb = on && rcp_ok(tbk);
           ok = ok && (onb || s >= ph.nsys);   // the backward one too
           const double tb = onb ? rcp_f64(tbk) : 0.0;
-          ld_at(dcol, LD_TAU + NSYS + s) = tb;
-          ls_at(col, LS_LAW + NSYS + s) = f64_to_f32(tb);
+          dcol(LD_TAU + NSYS + s) = tb;
+          col(LS_LAW + NSYS + s) = f64_to_f32(tb);
         }
       }
     } else {
 #pragma unroll 4
-      for (int s = 0; s < 3 * NSYS; s++) ls_at(col, LS_LAW + s) = f64_to_f32(io.slip(s));
+      for (int s = 0; s < 3 * NSYS; s++) col(LS_LAW + s) = f64_to_f32(io.slip(s));
     }
     const SolveF32 o = solve_f32<LS_FAST, LAW, GEN, true>(lc, pf, col, 0.0f, ref2, f64_to_f32(h), f64_to_f32(dh),
                                                           xf, edf);
@@ -313,7 +315,7 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
         for (int j = 0; j < 5; j++) {
           double a = 0;
 #pragma unroll
-          for (int i = 0; i < 5; i++) a += ld_at(dcol, LD_Q + i * 5 + j) * x[i];
+          for (int i = 0; i < 5; i++) a += dcol(LD_Q + i * 5 + j) * x[i];
           t[j] = a;
         }
         io.stot(nc, ph, t, u, dcol);
@@ -321,7 +323,7 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
         for (int i = 0; i < 5; i++) {
           double a = c[i] + nc.dt * ed[i];
 #pragma unroll
-          for (int j = 0; j < 5; j++) a += ld_at(dcol, LD_Q + i * 5 + j) * u[j];
+          for (int j = 0; j < 5; j++) a += dcol(LD_Q + i * 5 + j) * u[j];
           rf[i] = -f64_to_f32(a);
           xf[i] = f64_to_f32(x[i]);
         }
@@ -397,7 +399,7 @@ float2 g[NSYS / 2];
     double a = 0, b = 0;
 #pragma unroll
     for (int i = 0; i < 5; i++) {
-      const double q = ld_at(dcol, LD_Q + i * 5 + j);
+      const double q = dcol(LD_Q + i * 5 + j);
       a += q * x[i];
       b += q * ed[i];
     }
@@ -472,11 +474,11 @@ struct FieldIo {
     for (int i = 0; i < 15; i++) S[i] = etf[ET_STOT + i];
   }
   __device__ __forceinline__ void stot(const NewtonConst&, const PhaseConst&, const double (&t)[5], double (&u)[5],
-                                       double*) const {
+                                       const DCol&) const {
     symv5_packed(et + ET_STOT, t, u);
   }
   __device__ __forceinline__ void sel(const NewtonConst&, const PhaseConst&, const double (&t)[5], double (&u)[5],
-                                      double*) const {
+                                      const DCol&) const {
     symv5_packed(et + ET_SEL, t, u);
   }
   __device__ __forceinline__ void full(const NewtonConst&, const PhaseConst& ph, FullIo& o) const {
@@ -486,14 +488,14 @@ struct FieldIo {
 };
 
 template <int LAW, bool GEN>
-__global__ void __launch_bounds__(LS_NT, 6) newton_f64_kernel(const __grid_constant__ NewtonConst nc,
+__global__ void __launch_bounds__(F64_NT, 6) newton_f64_kernel(const __grid_constant__ NewtonConst nc,
                                                               const __grid_constant__ LocalConst lc,
                                                               const __grid_constant__ Fields<double> f,
                                                               double* __restrict__ partials, IterIn it) {
   if (!is_live(it)) return;
   extern __shared__ __align__(16) float ls_sm[];
-  float* col = ls_sm + threadIdx.x;
-  double* dcol = reinterpret_cast<double*>(ls_sm + LS_NT * ls_rows<LAW, GEN>()) + threadIdx.x;
+  const FCol col{ls_sm + threadIdx.x};
+  const DCol dcol{reinterpret_cast<double*>(ls_sm + F64_NT * ls_rows<LAW, GEN>()) + threadIdx.x};
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long P = f.nv;
   double acc[NPART];
@@ -526,7 +528,7 @@ __global__ void __launch_bounds__(LS_NT, 6) newton_f64_kernel(const __grid_const
       }
     }
   }
-  newton_block_sums<double, GEN>(acc, dcol, partials);
+  newton_block_sums<double, GEN, F64_NT>(acc, dcol, partials);
 }
 
 
@@ -601,25 +603,25 @@ struct ArrayIo {
       }
   }
   __device__ __forceinline__ void sel(const NewtonConst&, const PhaseConst&, const double (&t)[5], double (&u)[5],
-                                      double* dcol) const {
+                                      const DCol& dcol) const {
     double y[5];
 #pragma unroll
     for (int k = 0; k < 5; k++) {
       double a = 0;
 #pragma unroll
-      for (int j = 0; j < 5; j++) a += ld_at(dcol, LD_Q + k * 5 + j) * t[j];
+      for (int j = 0; j < 5; j++) a += dcol(LD_Q + k * 5 + j) * t[j];
       y[k] = a * ph.s_xt[k];
     }
 #pragma unroll
     for (int j = 0; j < 5; j++) {
       double a = 0;
 #pragma unroll
-      for (int k = 0; k < 5; k++) a += ld_at(dcol, LD_Q + k * 5 + j) * y[k];
+      for (int k = 0; k < 5; k++) a += dcol(LD_Q + k * 5 + j) * y[k];
       u[j] = a;
     }
   }
   __device__ __forceinline__ void stot(const NewtonConst& nc, const PhaseConst& p, const double (&t)[5],
-                                       double (&u)[5], double* dcol) const {
+                                       double (&u)[5], const DCol& dcol) const {
     sel(nc, p, t, u, dcol);
 #pragma unroll
     for (int i = 0; i < 5; i++)
@@ -643,7 +645,7 @@ struct ArrayIo {
 
 // one thread per point; block_iters receives each block's Newton steps
 template <bool GEN>
-__global__ void __launch_bounds__(LS_NT, 6) local_solve_kernel(const __grid_constant__ NewtonConst nc,
+__global__ void __launch_bounds__(F64_NT, 6) local_solve_kernel(const __grid_constant__ NewtonConst nc,
                                                                const __grid_constant__ LocalConst lc, long long n,
                                                                double* sig, const double* __restrict__ epsp,
                                                                const double* __restrict__ strain,
@@ -652,9 +654,9 @@ __global__ void __launch_bounds__(LS_NT, 6) local_solve_kernel(const __grid_cons
                                                                double* __restrict__ edot, double* __restrict__ err,
                                                                double* __restrict__ block_iters) {
   extern __shared__ __align__(16) float ls_sm[];
-  __shared__ int steps[LS_NT / 32];
-  float* col = ls_sm + threadIdx.x;
-  double* dcol = reinterpret_cast<double*>(ls_sm + LS_NT * ls_rows<0, GEN>()) + threadIdx.x;
+  __shared__ int steps[F64_NT / 32];
+  const FCol col{ls_sm + threadIdx.x};
+  const DCol dcol{reinterpret_cast<double*>(ls_sm + F64_NT * ls_rows<0, GEN>()) + threadIdx.x};
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int it = 0;
   if (v < n) {
@@ -712,7 +714,7 @@ cudaError_t launch_local_solve(const NewtonConst& nc, long long n, double* sig, 
 // process exits.  Calls that overlap on the GPU share it and race.
 namespace {
 constexpr long long NOALLOC_MAX_VOXELS = 1LL << 20;
-constexpr int NOALLOC_MAX_BLOCKS = (int)(NOALLOC_MAX_VOXELS / LS_NT);   // smaller blocks only below 2^17 points
+constexpr int NOALLOC_MAX_BLOCKS = (int)(NOALLOC_MAX_VOXELS / F64_NT);   // smaller blocks only below 2^17 points
 static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_MAX_BLOCKS + 1];
 
 __global__ void noalloc_total_kernel(double* scratch, int nblocks) {
