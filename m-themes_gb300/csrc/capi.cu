@@ -596,7 +596,6 @@ extern "C" mth_status mth_create(const mth_params* p, mth_ctx** out) {
     }                                                                                              \
   } while (0)
   CKC(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
-  CKC(prepare_newton_kernels());
   // failure-path test hook: MTH_TEST_FAIL_TILE_WAIT=1 makes the tile passes'
   // first waits report a time-out (steps return MTH_ERR_TIMEOUT); every
   // context creation sets the device's hook from the environment

@@ -200,8 +200,6 @@ cudaError_t launch_newton_f64(const NewtonConst& nc, const Fields<double>& f, do
                               cudaStream_t st, int law);
 int newton_threads(long long nv, bool fp64);
 int newton_blocks(long long nv, bool fp64);
-// kernel attributes the Newton launches need, set on the current device
-cudaError_t prepare_newton_kernels();
 cudaError_t launch_end_step(int mixed, const NewtonConst& nc, const void* fields, const double anti_uniform[3],
                             int do_orient, int do_harden, double* partials, int nblocks, cudaStream_t st, int law = 0);
 cudaError_t launch_setup(int mixed, const NewtonConst& nc, const void* fields, const double* euler,

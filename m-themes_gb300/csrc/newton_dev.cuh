@@ -809,18 +809,4 @@ inline bool plain_phase(const NewtonConst& nc, const LocalConst& lc) {
   return nc.ph1_only && nc.ph[0].tau_back_minus_fwd == 0.0 && lc.ph[0].nm1 > 0;
 }
 
-// the opt-in above 48 KB of shared memory per block, once per device (also
-// done by prepare_newton_kernels when a context is created, so that no
-// attribute call falls inside a stream capture)
-template <typename K>
-cudaError_t smem_opt_in(K k, size_t bytes, bool (&set)[64]) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev >= 0 && dev < 64 && set[dev]) return cudaSuccess;
-  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) set[dev] = true;
-  return e;
-}
-
 }  // namespace mth

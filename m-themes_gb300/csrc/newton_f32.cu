@@ -226,6 +226,7 @@ template <int SOLVE, int LAW, bool GEN, int MINB>
 static cudaError_t launch_f32(const LocalConst& lc, const NewtonConst& nc, const Fields<float>& f, double* partials,
                               const IterIn& it, cudaStream_t st) {
   const int nt = newton_threads(f.nv, false);
+  static_assert(sizeof(float) * F32_NT * ls_rows<LAW, GEN>() <= 47 * 1024, "no opt-in above 48 KB is made");
   return launch_chain(newton_f32_kernel<SOLVE, LAW, GEN, MINB>, dim3(newton_blocks(f.nv, false)), dim3(nt),
                       sizeof(float) * F32_NT * ls_rows<LAW, GEN>(), st, it.pdl, lc, nc, f, partials, it);
 }

@@ -77,7 +77,11 @@ constexpr int LD_Q = 0, LD_TAU = 25;
 template <int LAW, bool GEN>
 __host__ __device__ constexpr int ld_rows() { return LD_TAU + (LAW == 1 ? 0 : GEN ? 2 * NSYS : NSYS); }
 template <int LAW, bool GEN>
-constexpr size_t f64_smem() { return (size_t)F64_NT * (4 * ls_rows<LAW, GEN>() + 8 * ld_rows<LAW, GEN>()); }
+constexpr size_t f64_smem() {
+  constexpr size_t b = (size_t)F64_NT * (4 * ls_rows<LAW, GEN>() + 8 * ld_rows<LAW, GEN>());
+  static_assert(b <= 47 * 1024, "no opt-in to more than 48 KB of shared memory is made");
+  return b;
+}
 
 // rates (crystal axes) at x in FP64
 template <int LAW, bool GEN, typename IO>
@@ -533,23 +537,8 @@ __global__ void __launch_bounds__(F64_NT, 6) newton_f64_kernel(const __grid_cons
 
 
 template <int LAW, bool GEN>
-static cudaError_t f64_opt_in() {
-  static bool set[64] = {};
-  return smem_opt_in(newton_f64_kernel<LAW, GEN>, f64_smem<LAW, GEN>(), set);
-}
-cudaError_t prepare_newton_kernels() {
-  cudaError_t e = f64_opt_in<0, false>();
-  if (e == cudaSuccess) e = f64_opt_in<0, true>();
-  if (e == cudaSuccess) e = f64_opt_in<1, false>();
-  if (e == cudaSuccess) e = f64_opt_in<1, true>();
-  return e;
-}
-
-template <int LAW, bool GEN>
 static cudaError_t launch_f64(const NewtonConst& nc, const LocalConst& lc, const Fields<double>& f, double* partials,
                               const IterIn& it, cudaStream_t st) {
-  cudaError_t e = f64_opt_in<LAW, GEN>();
-  if (e != cudaSuccess) return e;
   return launch_chain(newton_f64_kernel<LAW, GEN>, dim3(newton_blocks(f.nv, true)), dim3(newton_threads(f.nv, true)),
                       f64_smem<LAW, GEN>(), st, it.pdl, nc, lc, f, partials, it);
 }
@@ -690,16 +679,11 @@ cudaError_t launch_local_solve(const NewtonConst& nc, long long n, double* sig, 
   LocalConst lc;
   fill_local(nc, true, lc);
   for (int k = 0; k < 5; k++) lc.s_xt[k] = (float)nc.ph[0].s_xt[k];
-  static bool set0[64] = {}, set1[64] = {};
   const int nb = newton_blocks(n, true), nt = newton_threads(n, true);
   if (nc.ph[0].tau_back_minus_fwd == 0.0 && lc.ph[0].nm1 > 0) {
-    cudaError_t e = smem_opt_in(local_solve_kernel<false>, f64_smem<0, false>(), set0);
-    if (e != cudaSuccess) return e;
     local_solve_kernel<false><<<nb, nt, f64_smem<0, false>(), st>>>(nc, lc, n, sig, epsp, strain, rot, crss, edot, err,
                                                                     block_iters);
   } else {
-    cudaError_t e = smem_opt_in(local_solve_kernel<true>, f64_smem<0, true>(), set1);
-    if (e != cudaSuccess) return e;
     local_solve_kernel<true><<<nb, nt, f64_smem<0, true>(), st>>>(nc, lc, n, sig, epsp, strain, rot, crss, edot, err,
                                                                   block_iters);
   }
