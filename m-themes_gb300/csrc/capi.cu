@@ -767,10 +767,9 @@ extern "C" mth_status mth_destroy(mth_ctx* c) {
 static const int* plain_in(const mth_ctx* c) { return c->plain_step ? &c->bk_d->plain : nullptr; }
 IterIn iter_in(const mth_ctx* c) { return IterIn{c->add_d, c->live_d, c->in_batch ? 0 : c->pdl, plain_in(c)}; }
 
-// gated: the kernel follows the live flag (inside a batch graph)
 mth_status launch_reduce(mth_ctx* c, int width) {
   LAUNCH(K_REDUCE, 8.0 * width * (c->nblocks + 1),
-         launch_reduce_partials(c->partials, c->nblocks, width, c->red, IterIn{nullptr, nullptr}, c->st));
+         launch_reduce_partials(c->partials, c->nblocks, width, c->red, c->st));
   return MTH_OK;
 }
 

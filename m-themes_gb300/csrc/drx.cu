@@ -1242,7 +1242,8 @@ cudaError_t launch_pf_relax(const int dims[3], const int* grain, const T* rho, i
   const size_t tsm = sizeof(T) * PF_TB * PF_HN;
   PF_CK(cudaFuncSetAttribute(pf_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
   // the update's rows per 128-thread block, and the words of a row's bitmaps:
-  // none (the walk along the row) where they would pass 48 KB, z lines over 1408
+  // none (the walk along the row) where they would pass 47 KB: z lines over 1472,
+  // and lines of 5 voxels or fewer, of which a block takes 25 or more
   const int uper = dims[2] >= 128 ? 1 : 128 / dims[2];
   int uwords = (dims[2] + 31) / 32;
   size_t usm = sizeof(int) * (size_t)uper * PF_RH * (1 + uwords);

@@ -362,8 +362,7 @@ cudaError_t launch_disgrad_to_host(int mixed, const void* strain, const void* sk
 // skew += u + wspin per voxel, (W21, W02, W10) planes
 cudaError_t launch_disgrad_skew(int mixed, const void* wspin, void* skew, long long P, const double u[3],
                                 cudaStream_t st);
-cudaError_t launch_reduce_partials(const double* partials, int nblocks, int width, double* out, const IterIn& it,
-                                   cudaStream_t st);
+cudaError_t launch_reduce_partials(const double* partials, int nblocks, int width, double* out, cudaStream_t st);
 
 // the end of an iteration on the device (book.cu, book.cuh): the Newton
 // kernels' rows summed into red (NPART) and, with b, the bookkeeping; scratch:

@@ -425,8 +425,7 @@ cudaError_t launch_to_host_layout(int mixed, const void* src, long long P, int n
 // dependent ones.
 constexpr int RED_NT = 1024;   // 32 warps: the second shuffle stage sums one value per warp
 __global__ void __launch_bounds__(RED_NT) reduce_partials_kernel(const double* __restrict__ partials, int nblocks,
-                                                                 int width, double* __restrict__ out, IterIn it) {
-  if (!is_live(it)) return;
+                                                                 int width, double* __restrict__ out) {
   __shared__ double sm[RED_NT / 32];
   for (int w = blockIdx.x; w < width; w += gridDim.x) {
     double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
@@ -454,10 +453,9 @@ __global__ void __launch_bounds__(RED_NT) reduce_partials_kernel(const double* _
   }
 }
 
-cudaError_t launch_reduce_partials(const double* partials, int nblocks, int width, double* out, const IterIn& it,
-                                   cudaStream_t st) {
-  return launch_chain(reduce_partials_kernel, dim3(width), dim3(RED_NT), 0, st, it.pdl, partials, nblocks, width, out,
-                      it);
+cudaError_t launch_reduce_partials(const double* partials, int nblocks, int width, double* out, cudaStream_t st) {
+  reduce_partials_kernel<<<width, RED_NT, 0, st>>>(partials, nblocks, width, out);
+  return cudaGetLastError();
 }
 
 }  // namespace mth

@@ -27,14 +27,6 @@ __device__ __forceinline__ T pow_abs(T a, int ei, T ef) {
   return a > (T)0 ? (T)pow(a, ef) : (T)0;
 }
 
-// class-table row pointer of precision T
-template <typename T>
-__device__ __forceinline__ const T* cpick_ptr(const double* d, const float* f);
-template <>
-__device__ __forceinline__ const float* cpick_ptr<float>(const double*, const float* f) { return f; }
-template <>
-__device__ __forceinline__ const double* cpick_ptr<double>(const double* d, const float*) { return d; }
-
 // Flow rule in crystal axes at deviatoric stress x (5).  tauf: forward CRSS
 // per system; the backward CRSS is forward + tau_off.  Returns edot (5),
 // optional Hessian contribution D (15, packed upper triangle) and
@@ -194,17 +186,6 @@ __device__ __forceinline__ int pk(int i, int j) {  // packed upper-triangle inde
   return i * 5 - (i * (i - 1)) / 2 + (j - i);
 }
 
-template <typename T>
-__device__ __forceinline__ void symv5(const T* K, const T* x, T* y) {
-#pragma unroll
-  for (int i = 0; i < 5; i++) {
-    T s = 0;
-#pragma unroll
-    for (int j = 0; j < 5; j++) s += K[pk(i, j)] * x[j];
-    y[i] = s;
-  }
-}
-
 // 1/d for a positive normal FP64 pivot, without FP64-pipe work besides
 // three DFMA: the FP32 hardware reciprocal (rcp.approx.ftz.f32, within 1 ulp)
 // of d's mantissa m in [1, 2), truncated to 24 bits, gives 1/m to within
@@ -298,34 +279,20 @@ __device__ __forceinline__ bool ldl_solve5(const T* A, const T* b, T* x) {
   return true;
 }
 
-// LDL^T solve of a TF system in precision TL.  FP32 -> FP64 (and back):
-// the conversions by integer operations (f32_to_f64, f64_to_f32), as GB300
-// executes F2F conversions on its 1/64-rate FP64 pipe; the pivot
-// reciprocals with the quadratic step (the FP64 solve of an FP32 system is
-// rounded to FP32; 5 DFMA fewer per solve, the 400 Newton launches of the
-// 128^3 benchmark 2.3 % faster).
-template <typename TF, typename TL>
-__device__ __forceinline__ bool ldl_solve5_wide(const TF* H, const TF* b, TF* x) {
-  TL Hl[15], bl[5], pl[5];
-  if constexpr (sizeof(TF) == 4 && sizeof(TL) == 8) {
+// FP64 LDL^T solve of an FP32 system: the conversions by integer operations
+// (f32_to_f64, f64_to_f32), as GB300 executes F2F conversions on its 1/64-rate
+// FP64 pipe; the pivot reciprocals with the quadratic step (the result is
+// rounded to FP32; 5 DFMA fewer per solve).
+__device__ __forceinline__ bool ldl_solve5_wide(const float* H, const float* b, float* x) {
+  double Hl[15], bl[5], pl[5];
 #pragma unroll
-    for (int i = 0; i < 15; i++) Hl[i] = f32_to_f64(H[i]);
+  for (int i = 0; i < 15; i++) Hl[i] = f32_to_f64(H[i]);
 #pragma unroll
-    for (int i = 0; i < 5; i++) bl[i] = f32_to_f64(b[i]);
-    const bool ok = ldl_solve5<TL, true, true>(Hl, bl, pl);
+  for (int i = 0; i < 5; i++) bl[i] = f32_to_f64(b[i]);
+  const bool ok = ldl_solve5<double, true, true>(Hl, bl, pl);
 #pragma unroll
-    for (int i = 0; i < 5; i++) x[i] = f64_to_f32(pl[i]);
-    return ok;
-  } else {
-#pragma unroll
-    for (int i = 0; i < 15; i++) Hl[i] = (TL)H[i];
-#pragma unroll
-    for (int i = 0; i < 5; i++) bl[i] = (TL)b[i];
-    const bool ok = ldl_solve5<TL, true>(Hl, bl, pl);
-#pragma unroll
-    for (int i = 0; i < 5; i++) x[i] = (TF)pl[i];
-    return ok;
-  }
+  for (int i = 0; i < 5; i++) x[i] = f64_to_f32(pl[i]);
+  return ok;
 }
 
 // Result of one voxel solve.
@@ -616,20 +583,15 @@ __device__ __forceinline__ VoxelOut<TF> nw_finish(const NewtonState<TF>& s, cons
   return o;
 }
 
-// Local solve of one crystal voxel.  lam6/eps6/ep6: LT sample-frame inputs
-// (lambda = current stress, total strain, plastic strain); Q: sample->crystal
-// 5x5 of the current lattice orientation; et: elastic-class row (initial
-// orientation); tauf: forward CRSS.  Outputs sig6 (sample frame) and ed6
-// (plastic strain rate, sample frame).
-// TF: flow rule, residual, Hessian assembly, line search and frame
-// transforms; TL: precision of the Jacobian (Hessian) solve.  FP64 mode:
-// both double.  Mixed mode: TF = float, TL = double: the FP32-assembled 5x5
-// system is factored and solved in FP64 at every Newton step.  Mixed
-// root-FP64 mode (ROOT_ONLY): the FP64 solve only for the steps within
-// 1e-3 |lambda| of the root, which set the converged answer, and the FP32
-// factorisation for the large early steps, whose direction only has to be a
-// descent direction (GB300 issues FP64 at 1/64 of the FP32 rate).  Fast
-// mode: all float.
+// Local solve of one crystal voxel by the damped iteration in its plain order:
+// the FP64 mode's fallback and the iterations with a tight cap (solve_full), the
+// FP32 modes' irregular voxels and iterations in plain order (solve_steep).
+// lam6/eps6/ep6: LT sample-frame inputs (lambda = current stress, total strain,
+// plastic strain); et: elastic-class row (initial orientation).  Outputs sig6
+// (sample frame) and ed6 (plastic strain rate, sample frame).
+// TF: flow rule, residual, Hessian assembly, line search and frame transforms;
+// TL: precision of the 5x5 solve, at every step or (ROOT_ONLY) for the steps
+// within 1e-3 |lambda| of the root, with TF for the large early ones.
 // load(lam6, eps6, ep6, R, again) fills the voxel's inputs; it is called
 // at the start and again (again = true: loads the compiler may not merge
 // with the first) for the back-transform and the error norms, so neither
@@ -647,14 +609,10 @@ __device__ VoxelOut<TF> solve_voxel(const NewtonConst& nc, const PhaseConst& ph,
     if (k == 0) continue;
     TF p[5];
     bool ok;
-    if (sizeof(TL) > sizeof(TF) && (!ROOT_ONLY || s.near_root)) {
-      // Jacobian solve in TL (FP64) of the TF-assembled system: at every
-      // step, or (ROOT_ONLY) for the steps within 1e-3 |lambda| of the
-      // root, which set the converged answer
-      ok = ldl_solve5_wide<TF, TL>(H, mg, p);
-    } else {
+    if constexpr (sizeof(TL) > sizeof(TF))
+      ok = !ROOT_ONLY || s.near_root ? ldl_solve5_wide(H, mg, p) : ldl_solve5<TF>(H, mg, p);
+    else
       ok = ldl_solve5<TF>(H, mg, p);
-    }
     if (!nw_pass_b(s, nc, p, ok, mg)) break;
   }
   return nw_finish(s, nc, et, load, sig6, ed6);

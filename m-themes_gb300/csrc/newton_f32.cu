@@ -8,7 +8,7 @@ namespace mth {
 constexpr int F32_NT = 128;   // threads of the largest block
 
 __device__ __noinline__ bool solve5_f64(const float* H, const float* b, float* x) {
-  return ldl_solve5_wide<float, double>(H, b, x);
+  return ldl_solve5_wide(H, b, x);
 }
 
 // A voxel whose solve is not an ordinary one (local_solve.cuh), or with a CRSS

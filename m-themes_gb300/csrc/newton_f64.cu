@@ -227,7 +227,6 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
 #pragma unroll
         for (int i = 0; i < 6; i++) u[i] = ep[i] - u[i];
         rot_to_q_dev<double>(R, Q);
-        io.set_q(Q);
 #pragma unroll
         for (int i = 0; i < 25; i++) dcol(LD_Q + i) = Q[i];
         float Rf[9], Qf[25], S[15];
@@ -370,7 +369,7 @@ __device__ __forceinline__ void solve_f64(const NewtonConst& nc, const LocalCons
       prev = step;
       if (done) {
         // rates at the accepted iterate: + sum_s w_s m_s (m_s . p)
-float2 g[NSYS / 2];
+        float2 g[NSYS / 2];
         resolved2(pf, p, g);
         const float sc = LAW == 0 ? pf.gn : 1.0f;
 #pragma unroll
@@ -472,7 +471,6 @@ struct FieldIo {
   }
   __device__ __forceinline__ double slip(int s) const { return (LAW ? f.ddc : f.crss)[s * f.nv + v]; }
   __device__ __forceinline__ double shh() const { return et[ET_SEL_HH]; }
-  __device__ __forceinline__ void set_q(const double (&)[25]) {}
   __device__ __forceinline__ void s_packed(const LocalConst&, const SlipF&, const float (&)[25], float (&S)[15]) const {
 #pragma unroll
     for (int i = 0; i < 15; i++) S[i] = etf[ET_STOT + i];
@@ -575,7 +573,6 @@ struct ArrayIo {
   }
   __device__ __forceinline__ double slip(int s) const { return s < ph.nsys ? crss[NSYS * v + s] : 0.0; }
   __device__ __forceinline__ double shh() const { return ph.s_xt[5]; }
-  __device__ __forceinline__ void set_q(const double (&)[25]) {}
   __device__ __forceinline__ void s_packed(const LocalConst& lc, const SlipF&, const float (&Q)[25],
                                            float (&S)[15]) const {
     float s[5];
