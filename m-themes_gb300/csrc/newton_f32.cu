@@ -158,7 +158,21 @@ __global__ void __launch_bounds__(F32_NT, MINB) newton_f32_kernel(const __grid_c
           float2 xe[5], se[5];
 #pragma unroll
           for (int i = 0; i < 5; i++) xe[i] = make_float2(x[i], ed[i]);
-          dev_to_sample2(R, xe, se);
+          if constexpr (LAW == 0) {
+            dev_to_sample2(R, xe, se);
+          } else {
+            // Q^T x: two roundings fewer than T X T^T.  The sinh law's stress is off by
+            // 2.34e-7 from 64 bits with it and by 2.50e-7 without (96^3, three seeds; 17.9
+            // and 17.8 ms for 100 launches); the power law's by the same 2.1e-7 either way.
+            float Q[25];
+            rot_to_q_dev<float>(R, Q);
+#pragma unroll
+            for (int j = 0; j < 5; j++) {
+              se[j] = mul2(dup2(Q[j]), xe[0]);
+#pragma unroll
+              for (int i = 1; i < 5; i++) se[j] = fma2(dup2(Q[i * 5 + j]), xe[i], se[j]);
+            }
+          }
 #pragma unroll
           for (int i = 0; i < 5; i++) {
             ss[i] = se[i].x;
