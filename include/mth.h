@@ -86,7 +86,9 @@ typedef struct {
                                 ends when its last step is within it; in the mixed modes also
                                 when the next step is bounded within it (|gradient| over the
                                 smallest eigenvalue of the elastic Hessian base) */
-  int    newton_itmax;       /* <=0 selects 500 (src/evolution.c:105) */
+  int    newton_itmax;       /* <=0 selects 500 (src/evolution.c:105); below 50 the FP64 mode and
+                                the array solves keep every pass in FP64, which is several times
+                                slower: their FP32 start would spend part of so tight a cap */
   /* Phase-field / DRX block (src/io.c:71-90) */
   double pf_length_scale;    /* dx [m] */
   double pf_time_step;       /* dt of one PF substep [s] */
@@ -141,7 +143,10 @@ typedef struct {
   double e_vm, evmp, d_vm, dvmp, s_vm, s_vm1;
   double err_s, err_e;       /* final normalised errors */
   long long newton_iters;    /* local Newton iterations summed over voxels and Green iterations */
-  long long newton_failed;   /* voxel solves that hit the iteration cap */
+  long long newton_failed;   /* voxel solves that hit the iteration cap, or in the mixed modes met a
+                                pivot that is not positive (long first steps at a high exponent);
+                                they keep their iterate, and the fields are then not the
+                                converged ones: the FP64 mode converges on such volumes */
   int    n_new_grains;       /* DRX nuclei seeded this step */
   /* dislocation-density law: the dd.out columns after TIME and EVM
    * (src/evolution.c:1566-1569): volume averages of the per-system sums of

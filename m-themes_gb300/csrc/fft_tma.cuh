@@ -2,8 +2,8 @@
 // lengths with compile-time plans (MTH_TMA_SIZES).  Each pass asks only for
 // its own lengths: z for n2, y for n0 and n1, x + Green for n0; the others
 // (384, 512 and the like) take the shared-memory passes of fft_green.cu.  One
-// FP32 iteration of 72 x 54 x 108 (r2c / y / x + Green / c2r, us): 14 / 19 /
-// 16 / 14 here, 31 / 68 / 47 / 46 there; FP64 89 / 149 / 266 / 107 and 121 /
+// FP32 iteration of 72 x 54 x 108 (r2c / y / x + Green / c2r, us): 12 / 19 /
+// 16 / 15 here, 31 / 68 / 47 / 46 there; FP64 89 / 150 / 266 / 106 and 121 /
 // 204 / 344 / 135; of 18 x 24 x 36 FP32 8 / 13 / 9 / 8 and 13 / 31 / 21 / 17.
 //
 // Same passes and results as fft_green.cu (src/evolution.c:1361-1405), laid

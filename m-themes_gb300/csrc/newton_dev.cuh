@@ -1,6 +1,6 @@
 // newton_dev.cuh -- device code shared by the local-solve kernels
 // (newton_f32.cu, newton_f64.cu) and the end-of-step kernel (newton.cu): the
-// flow rules and the damped FP64 Newton iteration, the block sums, and the
+// flow rules and the damped Newton iteration in plain order, the block sums, and the
 // constants a launch fills.
 #pragma once
 #include <cmath>

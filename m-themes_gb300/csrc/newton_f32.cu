@@ -226,8 +226,8 @@ __global__ void __launch_bounds__(F32_NT, MINB) newton_f32_kernel(const __grid_c
   newton_block_sums<float, GEN, F32_NT>(acc, col, partials);
 }
 
-// Blocks of 128 threads per SM the kernels are compiled for.  100 launches,
-// ms: 128^3 33.3 with 4 (128 registers), 35.9 with 3, 36.1 with 5, 39.9 with 6;
+// Blocks of 128 threads per SM the kernels are compiled for.  100 launches of
+// an earlier state, ms: 128^3 33.3 with 4 (128 registers), 35.9 with 3, 36.1 with 5, 39.9 with 6;
 // dislocation-density law at 96^3 17.2 with 4, 19.0 with 3, 23.4 with 5.
 #ifndef MTH_F32_MINB
 #define MTH_F32_MINB 4
