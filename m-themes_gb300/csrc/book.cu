@@ -96,7 +96,7 @@ __device__ __forceinline__ bool book_end(IterBook& b, const double* red, BookTmp
   else if (lane == 13) b.it_nbad += (long long)red[15];
   else if (lane == 14) b.err_s = red[0] * b.wgt;
   else if (lane == 15) b.err_e = red[1] * b.wgt;
-  else if (lane == 16 && b.it_iter == 1 && !(red[15] > 0.0)) b.plain = 0;
+  else if (lane == 16 && b.plain == 1 && b.it_iter == 1 && !(red[15] > 0.0)) b.plain = 0;
   __syncwarp();
   if (lane < 18) {   // v2t: sig_avg (lanes 0-8), sig_avg1 (lanes 9-17)
     const int e = lane % 9;

@@ -30,11 +30,13 @@ struct IterBook {
   // The FP32 modes' iterations in plain order.  Where local solves fail (a high
   // exponent at a low CRSS, newton_f32.cu) the rounding of every operation of
   // the iteration decides which ones do, and the stress fields differ by percents
-  // from one rounding to another.  The first iteration of a volume, or after a
-  // step with failures, therefore runs every solve by solve_steep and the
-  // transforms and Green operator in their plain order, and so do the step's
-  // other iterations if a solve fails in it; without failures the order no longer
-  // matters (1e-7) and the faster one is taken from the second iteration on.
+  // from one rounding to another.  The first iteration of a volume therefore
+  // runs every solve by solve_steep and the transforms and Green operator in
+  // their plain order (1), and so do the step's other iterations if a solve fails
+  // in it and those of a step after one with failures (2), where single voxels
+  // still have long steps (else up to 1.6e-3 off in one or two of them).  Without
+  // failures the order no longer matters (1e-7) and the faster one is taken from
+  // the second iteration on.
   int plain;
   // state
   double ddg[3][3], ddg_acum[3][3], ddg_applied[3][3], sig_avg[3][3], sig_avg1[3][3];
@@ -154,7 +156,7 @@ MTH_HD inline bool book_finish(IterBook& b, const double* red, int npart) {
     }
   b.it_nit += (long long)red[14];
   b.it_nbad += (long long)red[15];
-  if (b.it_iter == 1 && !(red[15] > 0.0)) b.plain = 0;
+  if (b.plain == 1 && b.it_iter == 1 && !(red[15] > 0.0)) b.plain = 0;
   b.err_s = red[0] * b.wgt;
   b.err_e = red[1] * b.wgt;
   book_smacro(b, red);

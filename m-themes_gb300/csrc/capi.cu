@@ -1237,7 +1237,7 @@ mth_status step_begin(mth_ctx* c) {
   b.err = c->p.err;
   b.e_vm = c->e_vm;
   b.iter_max = c->p.iter_max;
-  c->plain_step = c->plain_next && !c->nc.flow_off && c->mixed && !c->dd;
+  c->plain_step = c->nc.flow_off || !c->mixed || c->dd ? 0 : c->plain_next;
   b.plain = c->plain_step;
   b.nan = 0;
   memset(b.ddg, 0, sizeof(b.ddg));
@@ -1370,7 +1370,7 @@ mth_status step_end(mth_ctx* c, mth_step_report* rep) {
   }
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++) c->disgrad_avg[i][j] = c->disgrad_avg_t[i][j] + c->udot[i][j] * dt;
-  if (!c->nc.flow_off) c->plain_next = c->bk.it_nbad > 0;
+  if (!c->nc.flow_off) c->plain_next = c->bk.it_nbad > 0 ? 2 : 0;
   c->istep++;
   return MTH_OK;
 }

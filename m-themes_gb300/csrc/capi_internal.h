@@ -116,8 +116,8 @@ struct mth_ctx {
   bool host_book;     // bookkeeping on the host after every iteration instead (test hook)
   int pdl;            // programmatic dependent launches along the iteration's kernels
   int istep;
-  int plain_next;     // the next step's first iteration runs in plain order (IterBook::plain)
-  int plain_step;     // the step in progress may hold such iterations
+  int plain_next;     // the next step's IterBook::plain: 1 a volume's first step, 2 after failures
+  int plain_step;     // that of the step in progress when it began
   int uploaded;
   // dynamic recrystallisation
   int drx;
