@@ -59,3 +59,18 @@ def test_batch_members(gold):
             for i, seed in ((0, 11), (2, 4)):
                 _check(gold, "mixed_%d" % seed, step, reps[i], b.field(i, "sig"))
             assert reps[1]["newton_failed"] == 0
+
+
+@pytest.mark.parametrize("tau0,seed", [(12.0, 4), (12.5, 34)])
+def test_step_after_failures(tau0, seed):
+    """The step after one with failures stays in plain order: the 64 voxels that come out most
+    different (by up to 3e-4 of the field's rms) when it leaves that order after its first
+    iteration.  The order keeps the bits; the fields' 2e-5 is allowed."""
+    gold = np.load(os.path.join(GOLDEN, "steep_second_steps.npz"))
+    cfg = synth.Config(cell_dim=(32, 32, 16), n_grains=20, n_steps=2, seed=seed, iter_max=20,
+                       material=synth.Material(nrs=20.0, tau0f=tau0, tau0b=tau0))
+    with Solver(capi.params_from_config(cfg, precision=capi.MTH_MIXED_FAST), *synth.microstructure(cfg)) as s:
+        assert s.step()["newton_failed"] > 0
+        s.step()
+        sig = np.asarray(s.field("sig"))[gold["voxels_%d" % seed]][:, [0, 1, 2, 4, 5, 8]]
+    assert np.abs(sig - gold["sig_%d" % seed]).max() < FP32_FIELD * gold["rms_%d" % seed]
